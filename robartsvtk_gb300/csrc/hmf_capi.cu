@@ -300,7 +300,7 @@ int plan_flow(hmf_ctx* c, int zchunk) {
     F.G.vol = V.vol;
     const int nx = (V.vx + hmf::kTmaMaxOutX - 1) / hmf::kTmaMaxOutX;
     const int ny = (V.vy + flow_max_out_y(c) - 1) / flow_max_out_y(c);
-    F.out_x = (V.vx + nx - 1) / nx;
+    F.out_x = ((V.vx + nx - 1) / nx + 1) & ~1;  // even: a thread owns two columns
     F.out_y = (V.vy + ny - 1) / ny;
     F.tiles_x = nx;
     F.zchunk = std::min(zchunk, V.vz);
@@ -522,6 +522,7 @@ int launch_flow_tma_items(hmf_ctx* c, const hmf::FlowVertexTMA* table, int parit
   hmf::FlowTmaParams fp;
   fp.step = c->step;
   fp.icc = 1.0f / c->cc;
+  fp.neg_zero = -0.0f;
   fp.parity = parity;
   fp.n_vertices = c->n - 1;
   fp.n_items = n_items;

@@ -117,45 +117,33 @@ struct TreeTable {
 };
 
 constexpr int kTmaBoxX = 36;   // box width: 16-byte aligned start plus 32 lanes plus 1
-constexpr int kTmaRows = 32;   // window rows
-constexpr int kTmaPlane = kTmaBoxX * kTmaRows;        // floats per staged array plane
-// Two rings.  The z flow of plane k+1 is needed one step early (the divergence
-// of plane k), everything else only in its own step, so the main ring (px, py,
-// sink, label, parent sink, smoothness) has 3 slots and the pz ring 4.  Plane
-// k + kTmaMainLead (main ring) and pz of plane k + 1 + kTmaPzLead are issued
-// in step k, after its first CTA barrier, kTmaMainLead / kTmaPzLead steps
-// before their first use.  The leads may rise to the slot counts (main) and
-// the slot count less one (pz); on a GB300 at 256^3 a lead of 3 on both rings
-// measured 0.9 % slower per iteration than 2, and 3 on either ring alone
-// within 0.2 %, so both stay at 2.
-constexpr int kTmaMainArrays = 6;
-constexpr int kTmaMainSlots = 3;
-constexpr int kTmaPzSlots = 4;
-constexpr int kTmaMainLead = 2;
-constexpr int kTmaPzLead = 2;
-static_assert(kTmaMainLead >= 1 && kTmaMainLead <= kTmaMainSlots, "main-ring lead");
-static_assert(kTmaPzLead >= 1 && kTmaPzLead <= kTmaPzSlots - 1, "pz-ring lead");
+// Rings of staged planes.  Plane k's px, py, sink, label and parent sink are
+// read in step k before its CTA barrier, so two slots carry a lead of two
+// steps: plane k + 2 is issued after that barrier into plane k's slot.  The
+// smoothness is read one step later and issued one plane behind, again in two
+// slots; pz of plane k + 1 is read in step k already, so pz runs one plane
+// ahead in three.  What step k needs -- main plane k, pz of plane k + 1,
+// smoothness of plane k - 1 -- completes on one mbarrier.
+constexpr int kTmaMainArrays = 5;
+constexpr int kTmaMainSlots = 2;
+constexpr int kTmaPzSlots = 3;
 constexpr int kTmaMaxOutX = 28;
 constexpr int kTmaMaxOutY = 27;
-constexpr int kTmaThreads = 256;
-constexpr int kTmaSmemBytes =
-                              (kTmaMainSlots * kTmaMainArrays + kTmaPzSlots) * kTmaPlane * 4 +
-                              (3 * 256 + 2 * 256) * 4 + 64;
-
-// Shape of flow_tma_kernel<W>: W warps of 4 register rows, a window of 32
-// columns x 4W rows (the TMA box is kTmaBoxX x 4W), 28 x (4W - 5) outputs.
-// W = 8: two CTAs per SM (~108 KB of shared memory each); W = 16: one CTA of
-// 16 warps per SM (~208 KB), half the halo rows per output.
+// Shape of flow_tma_kernel<W>: W warps, a window of 32 columns x 4W rows (the
+// TMA box is kTmaBoxX x 4W), 28 x (4W - 5) outputs.  A half-warp covers the 32
+// columns of two rows, two columns per lane.
 template <int W>
 struct FlowTmaShape {
   static constexpr int kRows = 4 * W;
+  static constexpr int kHalfWarps = 2 * W;
   static constexpr int kThreads = 32 * W;
   static constexpr int kPlane = kTmaBoxX * kRows;
   static constexpr int kMaxOutY = kRows - 5;
   static constexpr int kCtasPerSm = W <= 8 ? 2 : 1;
-  static constexpr int kSmemBytes = (kTmaMainSlots * kTmaMainArrays + kTmaPzSlots) * kPlane * 4 + 5 * kThreads * 4 + 64;
+  static constexpr int kPlanes = kTmaMainSlots * (kTmaMainArrays + 1) + kTmaPzSlots;
+  static constexpr int kSmemBytes = kPlanes * kPlane * 4 + 4 * 2 * kHalfWarps * 32 * 4 + 64;  // rings, exchange rows, mbarriers
 };
-static_assert(FlowTmaShape<8>::kSmemBytes == kTmaSmemBytes, "the 32-row shape keeps its layout");
+static_assert(kTmaPzSlots == kTmaMainSlots + 1, "the planes in flight");
 static_assert(FlowTmaShape<16>::kSmemBytes <= 227 * 1024, "the 64-row shape fits one SM's shared memory");
 
 struct FlowVertexTMA {  // 64-byte aligned through its CUtensorMap members
@@ -188,6 +176,7 @@ struct FlowItem {
 struct FlowTmaParams {
   float step;
   float icc;
+  float neg_zero;     // -0: the addend of packed multiplications (hmf_f32x2.cuh)
   int parity;
   int n_vertices;     // non-root vertices: units = n_vertices * n_items
   int n_items;        // work items of this launch (from `items`)
