@@ -25,6 +25,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <chrono>
 #include <climits>
 #include <cmath>
@@ -584,6 +585,23 @@ int tree_grid(hmf_ctx* c) {
   return (int)std::min<long long>(blocks, (long long)c->sm_count * 16);
 }
 
+// Grid of the kernels that take four voxels per thread (vol: elements).
+int quad_grid(long long vol, int sm_count) {
+  return (int)std::max<long long>(1, std::min<long long>((vol / 4 + 255) / 256, (long long)sm_count * 16));
+}
+
+// REF_CPU's iterations: a CC that is a power of two divides as its reciprocal
+// multiplies.
+void launch_refcpu(const hmf::TreeTable* table, const hmf::Geometry& G, int iterations, float cc, int sm_count,
+                   cudaStream_t s) {
+  int exponent = 0;
+  const int grid = quad_grid(G.vol, sm_count);
+  if (cc >= FLT_MIN && std::frexp(cc, &exponent) == 0.5f)
+    hmf::refcpu_kernel<true><<<grid, 256, 0, s>>>(table, G, iterations);
+  else
+    hmf::refcpu_kernel<false><<<grid, 256, 0, s>>>(table, G, iterations);
+}
+
 // The convergence log's device view (the arena of hmf_set_convergence_log).
 hmf::GapLog gap_view(const hmf_ctx* c, int t) {
   hmf::GapLog g{};
@@ -1127,11 +1145,8 @@ int do_init(hmf_ctx* c, cudaStream_t s, int) {
     ++c->launches;
     return HMF_OK;
   }
-  const size_t smem = (size_t)c->n * kTreeThreads * sizeof(float);
-  hmf::init_kernel<<<tree_grid(c), kTreeThreads, smem, s>>>(c->d_tree, c->geo, c->d_smooth_list,
-                                                           c->n_smooth_list,
-                                                           c->semantics == HMF_SEMANTICS_REF_CPU,
-                                                           c->d_error);
+  hmf::init_kernel<<<quad_grid(c->geo.vol, c->sm_count), 256, 0, s>>>(c->d_tree, c->geo, c->d_smooth_list, c->n_smooth_list,
+                                               c->semantics == HMF_SEMANTICS_REF_CPU, c->d_error);
   CK(cudaGetLastError(), "init_kernel launch");
   ++c->launches;
   return HMF_OK;
@@ -1140,7 +1155,7 @@ int do_init(hmf_ctx* c, cudaStream_t s, int) {
 int do_flow(hmf_ctx* c, cudaStream_t s, int parity) { return launch_flow(c, parity, s); }
 int do_tree(hmf_ctx* c, cudaStream_t s, int) { return launch_tree(c, s); }
 int do_refcpu(hmf_ctx* c, cudaStream_t s, int) {
-  hmf::refcpu_kernel<<<tree_grid(c), kTreeThreads, 0, s>>>(c->d_tree, c->geo, c->iterations);
+  launch_refcpu(c->d_tree, c->geo, c->iterations, c->cc, c->sm_count, s);
   CK(cudaGetLastError(), "refcpu_kernel launch");
   ++c->launches;
   return HMF_OK;
@@ -1156,9 +1171,6 @@ int configure_kernels(hmf_ctx* c) {
   const int tree_smem = 3 * hmf::kMaxVertices * kTreeThreads * (int)sizeof(float);
   CK(cudaFuncSetAttribute(hmf::tree_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tree_smem),
      "cudaFuncSetAttribute(tree_kernel)");
-  CK(cudaFuncSetAttribute(hmf::init_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          hmf::kMaxVertices * kTreeThreads * (int)sizeof(float)),
-     "cudaFuncSetAttribute(init_kernel)");
   CK(cudaFuncSetAttribute(hmf::flow_tma_kernel<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           hmf::FlowTmaShape<8>::kSmemBytes),
      "cudaFuncSetAttribute(flow_tma_kernel)");
@@ -1328,7 +1340,9 @@ int begin_solve_with(hmf_ctx* c, cudaStream_t user, Staged& staged, StateLoader 
   c->st_data = staged.data;
   c->st_smooth = staged.smooth;
   if (load) return load(c, s, arg);  // a continued solve: the caller's state replaces the initialisation
-  // flows of parity 0 start at zero
+  // flows of parity 0 start at zero (REF_CPU never writes any flow: they are
+  // zero since the context was made)
+  if (c->semantics == HMF_SEMANTICS_REF_CPU) return timed(c, 2, s, do_init, 0);
   const size_t bytes = (size_t)c->total * sizeof(float);
   for (int v = 0; v < c->n; ++v) {
     if (v == c->root) continue;
@@ -2059,9 +2073,6 @@ int noalloc_setup(int device, unsigned char** out) {
   NCK(cudaFuncSetAttribute(hmf::tree_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            3 * hmf::kMaxVertices * kTreeThreads * (int)sizeof(float)),
       "cudaFuncSetAttribute(tree_kernel)");
-  NCK(cudaFuncSetAttribute(hmf::init_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           hmf::kMaxVertices * kTreeThreads * (int)sizeof(float)),
-      "cudaFuncSetAttribute(init_kernel)");
   *out = static_cast<unsigned char*>(p);
   return HMF_OK;
 }
@@ -2320,11 +2331,11 @@ extern "C" int hmf_solve_noalloc(int vx, int vy, int vz, const int* parent, int 
   // initialisation and iterations, as hmf_solve queues them
   const long long tblocks = (G.vol + kTreeThreads - 1) / kTreeThreads;
   const int tgrid = (int)std::min<long long>(tblocks, (long long)sm_count * 16);
-  hmf::init_kernel<<<tgrid, kTreeThreads, (size_t)t.n * kTreeThreads * sizeof(float), s>>>(
-      d_tree, G, d_smooth_list, n_distinct, semantics == HMF_SEMANTICS_REF_CPU, d_error);
+  hmf::init_kernel<<<quad_grid(G.vol, sm_count), 256, 0, s>>>(d_tree, G, d_smooth_list, n_distinct,
+                                                             semantics == HMF_SEMANTICS_REF_CPU, d_error);
   NCK(cudaGetLastError(), "init_kernel launch");
   if (semantics == HMF_SEMANTICS_REF_CPU) {
-    hmf::refcpu_kernel<<<tgrid, kTreeThreads, 0, s>>>(d_tree, G, iterations);
+    launch_refcpu(d_tree, G, iterations, cc, sm_count, s);
     NCK(cudaGetLastError(), "refcpu_kernel launch");
   } else {
     hmf::FlowParams fp;

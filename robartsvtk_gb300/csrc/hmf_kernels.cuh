@@ -364,57 +364,71 @@ __global__ void __launch_bounds__(kTree4Threads) tree4_kernel(const TreeTable* _
 // flags negative data terms or smoothness values (the reference rejects
 // them, vtkHierarchicalMaxFlowSegmentation.cxx:434-438, :470-474).
 // ---------------------------------------------------------------------------
-__global__ void init_kernel(const TreeTable* __restrict__ table, const Geometry G,
-                            const float* const* __restrict__ smooth_list, int n_smooth,
-                            int cpu_min, int* __restrict__ error_flag) {
+//
+// Four voxels per thread: bound by the arrays it reads and writes once (labels
+// and sinks of every vertex, the leaves' data, the smoothness images).  A
+// branch's label is summed from its kids' labels read back by the thread that
+// wrote them.
+__global__ void __launch_bounds__(256) init_kernel(const TreeTable* __restrict__ table, const Geometry G,
+                                                   const float* const* __restrict__ smooth_list, int n_smooth,
+                                                   int cpu_min, int* __restrict__ error_flag) {
   __shared__ TreeTable T;
-  extern __shared__ float vals[];
   for (int i = threadIdx.x; i < (int)(sizeof(TreeTable) / 4); i += blockDim.x)
     reinterpret_cast<int*>(&T)[i] = reinterpret_cast<const int*>(table)[i];
   __syncthreads();
-  const int n = T.n, nb = blockDim.x, t = threadIdx.x;
-  float* U = vals;  // [n][nb]
-  const int root = n - 1;
+  const int root = T.n - 1;
   int bad = 0;
-  for (long long i = (long long)blockIdx.x * nb + t; i < G.vol; i += (long long)gridDim.x * nb) {
+  // kern_MinBuffers (CUDA_hierarchicalmaxflow.cu:489-499) or, for REF_CPU,
+  // minBuffer (vtkMaxFlowSegmentationUtilities.cxx:77-83); they differ only
+  // for NaN and signed zeros.
+  auto least = [&](float m, float d) { return cpu_min ? ((m > d) ? d : m) : ((m < d) ? m : d); };
+  const long long nq = G.vol / 4;  // rows are padded to a multiple of 4 floats
+  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += (long long)gridDim.x * blockDim.x) {
+    const long long i = q * 4;
     // pitch 0: several volumes of different pitches back to back, whose
     // padding columns are zero (never written), so every element is checked
-    const long long row = G.pitch ? i / G.pitch : 0;
-    const bool inside = G.pitch == 0 || (i - row * G.pitch) < G.vx;
-    float m = T.e[T.leaves[0]].data[i];
+    const int x = G.pitch ? (int)(i % G.pitch) : 0;
+    const int nin = G.pitch ? min(4, max(0, G.vx - x)) : 4;  // voxels of the quad inside the volume
+    auto negative = [&](float4 d) {
+      return (nin > 0 && d.x < 0.0f) || (nin > 1 && d.y < 0.0f) || (nin > 2 && d.z < 0.0f) || (nin > 3 && d.w < 0.0f);
+    };
+    float4 m = ld4(T.e[T.leaves[0]].data + i);
+#pragma unroll 4
     for (int j = 1; j < T.n_leaves; ++j) {
-      const float d = T.e[T.leaves[j]].data[i];
-      // kern_MinBuffers (CUDA_hierarchicalmaxflow.cu:489-499) or, for REF_CPU,
-      // minBuffer (vtkMaxFlowSegmentationUtilities.cxx:77-83); they differ
-      // only for NaN and signed zeros.
-      m = cpu_min ? ((m > d) ? d : m) : ((m < d) ? m : d);
+      const float4 d = ld4(T.e[T.leaves[j]].data + i);
+      m = make_float4(least(m.x, d.x), least(m.y, d.y), least(m.z, d.z), least(m.w, d.w));
     }
-    float cnt = 0.0f;
+    float4 cnt = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
     for (int j = 0; j < T.n_leaves; ++j) {
-      const int e = T.leaves[j];
-      const float d = T.e[e].data[i];
-      if (inside && d < 0.0f) bad = 1;
-      const float lab = (m == d) ? 1.0f : 0.0f;
-      U[e * nb + t] = lab;
-      cnt = cnt + lab;
+      const float4 d = ld4(T.e[T.leaves[j]].data + i);
+      if (negative(d)) bad = 1;
+      cnt.x = cnt.x + (m.x == d.x ? 1.0f : 0.0f);
+      cnt.y = cnt.y + (m.y == d.y ? 1.0f : 0.0f);
+      cnt.z = cnt.z + (m.z == d.z ? 1.0f : 0.0f);
+      cnt.w = cnt.w + (m.w == d.w ? 1.0f : 0.0f);
     }
-    for (int j = 0; j < T.n_leaves; ++j) {
-      const int e = T.leaves[j];
-      U[e * nb + t] = U[e * nb + t] / cnt;
-    }
-    for (int e = 0; e < root; ++e) {
+    const float4 one = make_float4(1.0f / cnt.x, 1.0f / cnt.y, 1.0f / cnt.z, 1.0f / cnt.w);
+    const float4 none = make_float4(0.0f / cnt.x, 0.0f / cnt.y, 0.0f / cnt.z, 0.0f / cnt.w);
+    for (int e = 0; e < root; ++e) {  // post-order: kids before their branch
       const TreeEntry& E = T.e[e];
-      if (E.n_kids) {
-        float acc = 0.0f;
-        for (int j = 0; j < E.n_kids; ++j) acc = acc + U[T.kids[E.first_kid + j] * nb + t];
-        U[e * nb + t] = acc;
+      float4 u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (E.n_kids == 0) {
+        const float4 d = ld4(E.data + i);
+        u = make_float4(m.x == d.x ? one.x : none.x, m.y == d.y ? one.y : none.y, m.z == d.z ? one.z : none.z,
+                        m.w == d.w ? one.w : none.w);
+      } else {
+        for (int j = 0; j < E.n_kids; ++j) {
+          const float4 c = *reinterpret_cast<const float4*>(T.e[T.kids[E.first_kid + j]].label + i);
+          u = make_float4(u.x + c.x, u.y + c.y, u.z + c.z, u.w + c.w);
+        }
       }
-      E.label[i] = U[e * nb + t];
-      E.sink[i] = m;
+      st4(E.label + i, u);
+      st4(E.sink + i, m);
     }
-    T.e[root].sink[i] = m;
+    st4(T.e[root].sink + i, m);
     for (int j = 0; j < n_smooth; ++j)
-      if (inside && smooth_list[j][i] < 0.0f) bad = 1;
+      if (negative(ld4(smooth_list[j] + i))) bad = 1;
   }
   if (bad) atomicOr(error_flag, 1);
 }
@@ -428,30 +442,49 @@ __global__ void init_kernel(const TreeTable* __restrict__ table, const Geometry 
 // initial value, the minimum data term m.  What remains is, per leaf and voxel,
 //   sink = (m - 0) + u / CC;  sink = sink > D ? D : sink;  u += CC*((m - 0) - sink)
 // with no saturation, and branch labels that never change.  Every iteration of
-// a voxel is independent of its neighbours, so all iterations run in registers.
+// a voxel is independent of its neighbours and depends on its label alone, so
+// all iterations run in registers, and end early: an iteration that leaves a
+// label's bits as they were repeats itself for the rest.  (A label settles
+// once the sink is capped at m or the label is below the rounding of m, after
+// one or two iterations for most voxels; one that alternates between two
+// values runs to the end.)  A CC that is a power of two divides exactly as its
+// reciprocal multiplies (POW2).  What remains is one pass over the leaves'
+// data, labels and sinks; a quad is written only where a bit of it changed.
+// 192 x 160 x 144, 4 leaves, 200 iterations: 43 us, against 5.16 ms with every
+// iteration of every leaf divided out (the solve 145 us against 5.42 ms).
 // Called after init_kernel.
 // ---------------------------------------------------------------------------
-__global__ void refcpu_kernel(const TreeTable* __restrict__ table, const Geometry G, int iterations) {
+template <bool POW2>
+__global__ void __launch_bounds__(256) refcpu_kernel(const TreeTable* __restrict__ table, const Geometry G,
+                                                     int iterations) {
   __shared__ TreeTable T;
   for (int i = threadIdx.x; i < (int)(sizeof(TreeTable) / 4); i += blockDim.x)
     reinterpret_cast<int*>(&T)[i] = reinterpret_cast<const int*>(table)[i];
   __syncthreads();
-  const float cc = T.cc;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < G.vol;
-       i += (long long)gridDim.x * blockDim.x) {
+  const float cc = T.cc, icc = T.icc;
+  const long long nq = G.vol / 4;
+  auto step = [&](float m, float cap, float u, float& s) {
+    s = m + (POW2 ? u * icc : u / cc);
+    s = (s > cap) ? cap : s;
+    return u + cc * (m - s);
+  };
+  auto same = [](float a, float b) { return __float_as_uint(a) == __float_as_uint(b); };
+  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += (long long)gridDim.x * blockDim.x) {
+    const long long i = q * 4;
     for (int j = 0; j < T.n_leaves; ++j) {
       const TreeEntry& E = T.e[T.leaves[j]];
-      const float m = T.e[E.parent].sink[i];
-      const float cap = E.data[i];
-      float u = E.label[i];
-      float s = E.sink[i];
+      const float4 m = *reinterpret_cast<const float4*>(T.e[E.parent].sink + i), cap = ld4(E.data + i);
+      const float4 u0 = *reinterpret_cast<const float4*>(E.label + i), s0 = *reinterpret_cast<const float4*>(E.sink + i);
+      float4 u = u0, s = s0;
       for (int it = 0; it < iterations; ++it) {
-        s = (m - 0.0f) + u / cc;
-        s = (s > cap) ? cap : s;
-        u = u + cc * ((m - 0.0f) - s);
+        const float4 v = make_float4(step(m.x, cap.x, u.x, s.x), step(m.y, cap.y, u.y, s.y),
+                                     step(m.z, cap.z, u.z, s.z), step(m.w, cap.w, u.w, s.w));
+        const bool settled = same(v.x, u.x) && same(v.y, u.y) && same(v.z, u.z) && same(v.w, u.w);
+        u = v;
+        if (settled) break;
       }
-      E.label[i] = u;
-      E.sink[i] = s;
+      if (!(same(u.x, u0.x) && same(u.y, u0.y) && same(u.z, u0.z) && same(u.w, u0.w))) st4(E.label + i, u);
+      if (!(same(s.x, s0.x) && same(s.y, s0.y) && same(s.z, s0.z) && same(s.w, s0.w))) st4(E.sink + i, s);
     }
   }
 }
