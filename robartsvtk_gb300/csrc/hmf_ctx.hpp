@@ -242,6 +242,10 @@ int paged_copy_out(hmf_ctx* c, bool labels, int node, float* out, int where, voi
 void paged_free(hmf_ctx* c);
 size_t paged_bytes(const hmf_ctx* c);
 
+// hmf_dataterm.cu: the library's memory pool of the current device for per-call
+// scratch (null: none could be made; use cudaMalloc)
+cudaMemPool_t scratch_pool();
+
 // hmf_adjoint.cu
 void adjoint_free(hmf_ctx* c);
 size_t adjoint_bytes(const hmf_ctx* c);
