@@ -39,6 +39,7 @@
 
 #include "../../include/hmf.h"
 #include "hmf_ctx.hpp"
+#include "hmf_cell.cuh"
 #include "hmf_dag.cuh"
 #include "hmf_flow_tma.cuh"
 #include "hmf_kernels.cuh"
@@ -554,7 +555,70 @@ int launch_flow_tma_items(hmf_ctx* c, const hmf::FlowVertexTMA* table, int parit
   return HMF_OK;
 }
 
+// Small volumes run the cell kernels (hmf_cell.cuh): single label-tree volumes
+// of at most kCellVoxels voxel-vertices and 8 vertices, on the default flow
+// plan (a window, z chunk or units chosen by the caller keep the march), with
+// no convergence log and no stall requested of the copy pipelines.  The limit
+// lies where the two paths cross (time per iteration, three leaves: 24 x 20 x 16
+// 9.9 us against the march's 15.1, 40 x 36 x 28 11.8 against 20.9, 52 x 52 x 48
+// -- 389,000 -- 24.8 against 23.9, 64^3 35.9 against 31.3).
+constexpr long long kCellVoxels = 350000;
+
+bool cell_path(const hmf_ctx* c) {
+  return c->default_flow && c->pipeline && c->use_tma && c->tree_kind == 0 && !c->dag && c->vols.size() == 1 &&
+         c->n <= hmf::kSweepCellMax && !c->gap_on && c->stall_kind < 0 && c->semantics == HMF_SEMANTICS_REF_CUDA &&
+         c->total * (c->n - 1) <= kCellVoxels;
+}
+
+// A launch whose prologue may overlap the previous kernel of the stream (the
+// kernel waits for that one's results itself).
+template <class... Params, class... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, int threads, cudaStream_t s, Args... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
+int launch_flow_cell(hmf_ctx* c, int parity, cudaStream_t s) {
+  const auto& V = c->vols[0];
+  hmf::Geometry G{V.vx, V.vy, V.vz, V.pitch, V.plane, V.vol};
+  hmf::FlowParams fp{c->step, 1.0f / c->cc, 0, (V.vx + hmf::kCellX - 1) / hmf::kCellX};
+  const int tiles = fp.tiles_x * ((V.vy + hmf::kCellY - 1) / hmf::kCellY) * ((V.vz + hmf::kCellZ - 1) / hmf::kCellZ);
+  CK(launch_dependent(hmf::flow_cell_kernel, dim3(tiles, c->n - 1), hmf::kCellThreads, s, c->d_flow[parity], G, fp),
+     "flow_cell_kernel launch");
+  ++c->launches;
+  return HMF_OK;
+}
+
+int launch_sweep_cell(hmf_ctx* c, cudaStream_t s) {
+  const dim3 grid((unsigned)((c->geo.vol + hmf::kSweepCellThreads - 1) / hmf::kSweepCellThreads));
+  auto launch = [&](auto kernel) {
+    return launch_dependent(kernel, grid, hmf::kSweepCellThreads, s, c->d_tree, c->geo);
+  };
+  cudaError_t e = cudaErrorInvalidValue;
+  switch (c->n) {
+    case 2: e = launch(hmf::sweep_cell_kernel<2>); break;
+    case 3: e = launch(hmf::sweep_cell_kernel<3>); break;
+    case 4: e = launch(hmf::sweep_cell_kernel<4>); break;
+    case 5: e = launch(hmf::sweep_cell_kernel<5>); break;
+    case 6: e = launch(hmf::sweep_cell_kernel<6>); break;
+    case 7: e = launch(hmf::sweep_cell_kernel<7>); break;
+    case 8: e = launch(hmf::sweep_cell_kernel<8>); break;
+  }
+  CK(e, "sweep_cell_kernel launch");
+  ++c->launches;
+  return HMF_OK;
+}
+
 int launch_flow(hmf_ctx* c, int parity, cudaStream_t s) {
+  if (cell_path(c)) return launch_flow_cell(c, parity, s);
   if (c->use_tma) return launch_flow_tma(c, parity, s);
   // shared-memory ring flow kernel: single volumes only (checked at create)
   const auto& V = c->vols[0];
@@ -711,6 +775,7 @@ int launch_dag_sweep(hmf_ctx* c, cudaStream_t s) {
 
 int launch_tree(hmf_ctx* c, cudaStream_t s) {
   if (c->dag) return launch_dag_sweep(c, s);
+  if (cell_path(c)) return launch_sweep_cell(c, s);
   if (c->tree_kind == 0) return launch_tree_bulk_with(c, c->d_tree, s, c->gap_on, c->gap_t);
   if (c->tree_kind == 1) {
     const size_t smem4 = 4 * (size_t)c->n * hmf::kTree4Threads * sizeof(float4);
@@ -905,7 +970,7 @@ int record_gap_advance(hmf_ctx* c, int n_iter) {
 
 int capture(hmf_ctx* c, int n_iter, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
-  const bool slabs = pipeline_active(c);
+  const bool slabs = pipeline_active(c) && !cell_path(c);
   if (slabs)
     if (int rc = prepare_slabs(c, c->stream)) return rc;
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
@@ -1063,7 +1128,7 @@ int prepare_tables(hmf_ctx* c, cudaStream_t s, const Staged& in) {
   }
   CK(cudaMemcpyAsync(c->d_flow[0], fv.data(), sizeof(hmf::FlowVertex) * fv.size(), cudaMemcpyHostToDevice, s),
      "cudaMemcpyAsync(flow table)");
-  if (c->use_tma) {
+  if (c->use_tma && !cell_path(c)) {  // (the cell kernels need no tensor maps)
     std::vector<hmf::FlowVertexTMA>& tv = c->h_tma;
     tv.assign((size_t)nvol * nonroot, hmf::FlowVertexTMA{});
     for (int b = 0; b < nvol; ++b) {
@@ -1343,12 +1408,11 @@ int begin_solve_with(hmf_ctx* c, cudaStream_t user, Staged& staged, StateLoader 
   // flows of parity 0 start at zero (REF_CPU never writes any flow: they are
   // zero since the context was made)
   if (c->semantics == HMF_SEMANTICS_REF_CPU) return timed(c, 2, s, do_init, 0);
-  const size_t bytes = (size_t)c->total * sizeof(float);
   for (int v = 0; v < c->n; ++v) {
     if (v == c->root) continue;
+    // a vertex's three flows of one set lie back to back (allocate_state)
+    const size_t bytes = (char*)(c->fz[0][v] + c->total) - (char*)c->fx[0][v];
     CK(cudaMemsetAsync(c->fx[0][v], 0, bytes, s), "cudaMemsetAsync(flows)");
-    CK(cudaMemsetAsync(c->fy[0][v], 0, bytes, s), "cudaMemsetAsync(flows)");
-    CK(cudaMemsetAsync(c->fz[0][v], 0, bytes, s), "cudaMemsetAsync(flows)");
   }
   return timed(c, 2, s, do_init, 0);
 }
@@ -1530,13 +1594,14 @@ int solve_with(hmf_ctx* c, cudaStream_t user, StateLoader load, void* arg) {
       if (!rc) rc = capture(c, 1, &c->graph_one);
       // a pipelined solve replays several iterations per graph, so that the
       // pipeline drains (at a graph's end) rarely
-      if (!rc && pipeline_active(c)) rc = capture(c, kPipelineIterations, &c->graph_many);
+      if (!rc && (pipeline_active(c) || cell_path(c))) rc = capture(c, kPipelineIterations, &c->graph_many);
       if (rc) return rc;
     }
     // a DAG's last iteration runs fewer tasks: launched on its own
     const int graphed = c->dag ? std::max(0, c->iterations - 1) : c->iterations;
-    const long long per_iter = pipeline_active(c) ? 2LL * c->n_slabs : 2;
-    if (pipeline_active(c))
+    const bool slabs = pipeline_active(c) && !cell_path(c);
+    const long long per_iter = slabs ? 2LL * c->n_slabs : 2;
+    if (slabs)
       if (int rc2 = upload_slab_tables(c, s)) return rc2;
     int it0 = 0;
     if (c->graph_many)
@@ -1779,6 +1844,10 @@ int hmf_autotune(hmf_ctx* c, void* stream) {
   // those with 2 and 4 units (window-vertex marches) per CTA.
   c->timing = false;
   c->iterations = kTuneIterations;
+  // what is tuned is the march's plan, for contexts that run it: a small
+  // volume that the cell kernels take stays theirs
+  const bool saved_default = c->default_flow;
+  c->default_flow = false;
   auto time_plan = [&](int w, int z, int u, float* ms) -> int {
     c->flow_warps = w;
     c->flow_units = u;
@@ -1829,6 +1898,7 @@ int hmf_autotune(hmf_ctx* c, void* stream) {
   }
   c->iterations = saved_iters;
   c->timing = saved_timing;
+  c->default_flow = saved_default;
   c->solved = false;
   c->flow_warps = best.warps;
   c->flow_units = best.units;
@@ -1863,6 +1933,7 @@ int hmf_set_flow_window(hmf_ctx* c, int rows) {
   DeviceGuard dg(c->device);
   drop_graphs(c);
   c->flow_warps = rows == 64 ? 16 : 8;
+  c->default_flow = rows == 0;
   return plan_flow(c, default_zchunk(c));
 }
 
@@ -1876,6 +1947,7 @@ int hmf_set_flow_units(hmf_ctx* c, int units) {
   DeviceGuard dg(c->device);
   drop_graphs(c);  // the captured launches carry the grid
   c->flow_units = units ? units : 1;
+  c->default_flow = units == 0;
   return HMF_OK;
 }
 
@@ -1889,6 +1961,7 @@ int hmf_set_zchunk(hmf_ctx* c, int z) {
   drop_graphs(c);
   int maxz = 1;
   for (const auto& V : c->vols) maxz = std::max(maxz, V.vz);
+  c->default_flow = z == 0;
   return plan_flow(c, z ? std::min(z, maxz) : default_zchunk(c));
 }
 
