@@ -51,6 +51,12 @@ __device__ __forceinline__ F2 f2_mul(F2 a, F2 b, F2 neg_zero) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(neg_zero.v));
   return r;
 }
+// RN(a * b + c), one rounding
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
 // 8-byte aligned loads and stores of two neighbouring floats
 __device__ __forceinline__ F2 f2_ld(const float* p) { return F2{*reinterpret_cast<const unsigned long long*>(p)}; }
 __device__ __forceinline__ void f2_st(float* p, F2 a) { *reinterpret_cast<unsigned long long*>(p) = a.v; }

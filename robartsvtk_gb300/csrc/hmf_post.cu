@@ -63,10 +63,14 @@ constexpr size_t kEnergyBuffer = kEnergyTableBytes + sizeof(double) * (1 + hmf::
 // sums; null: allocated for this call.
 int launch_energy(hmf_ctx* c, const hmf::EnergyTable& tab, const hmf::Geometry& G, double* f0, double* f,
                   int n_nodes, cudaStream_t s, char* buffer) {
-  char* own = nullptr;
+  void* own = nullptr;
+  cudaMemPool_t pool = nullptr;
   if (!buffer) {
-    CK(cudaMalloc(&own, kEnergyBuffer), "cudaMalloc(energy buffer)");
-    buffer = own;
+    // from the library's pool, in stream order: cudaMalloc and cudaFree wait for the device
+    pool = scratch_pool();
+    CK(pool ? cudaMallocFromPoolAsync(&own, kEnergyBuffer, pool, s) : cudaMalloc(&own, kEnergyBuffer),
+       "cudaMalloc(energy buffer)");
+    buffer = static_cast<char*>(own);
   }
   hmf::EnergyTable* d_tab = reinterpret_cast<hmf::EnergyTable*>(buffer);
   double* d_sums = reinterpret_cast<double*>(buffer + kEnergyTableBytes);
@@ -92,18 +96,51 @@ int launch_energy(hmf_ctx* c, const hmf::EnergyTable& tab, const hmf::Geometry& 
       if (tab.parent_entry[k] >= 0) P.kids[tab.parent_entry[k]] |= 1u << k;
       P.sum_index[1 + k] = 1 + tab.vertex[k];
     }
+    P.neg_zero = -0.0f;
+    // pairs of voxels where every row and array starts 8-byte aligned (dense
+    // images of even width, and every array of a solver)
+    bool pairs = G.pitch % 2 == 0;
+    int slots = 0;
+    for (int k = 0; k < tab.n; ++k) P.slot[k] = tab.n_kids[k] == 0 || tab.parent_entry[k] >= 0 ? slots++ : -1;
+    const int pair_smem = slots * hmf::kEnergySlotFloats * hmf::kPostThreads * (int)sizeof(float);
+    for (int k = 0; k < tab.n; ++k)
+      for (const float* q : {tab.label[k], tab.data[k], tab.smooth[k]})
+        pairs = pairs && reinterpret_cast<uintptr_t>(q) % 8 == 0;
     auto launch = [&](auto kernel) { kernel<<<grid_of(kernel), hmf::kPostThreads, 0, s>>>(P, G, d_sums); };
+    // tiles in x and y, and z chunks for about two waves of CTAs (at least 4
+    // planes: a chunk reads a plane more on either side)
+    hmf::EnergyTiles T;
+    T.lanes_x = G.vx > 32 ? 32 : 16;
+    const int tile_rows = 2 * (hmf::kPostThreads / T.lanes_x);
+    T.tiles_x = (G.vx + 2 * T.lanes_x - 1) / (2 * T.lanes_x);
+    T.tiles_y = (G.vy + tile_rows - 1) / tile_rows;
+    auto launch_pairs = [&](auto kernel) {
+      int dev = 0, sms = 148, per = 1;
+      if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               hmf::kEnergyRegMax * hmf::kEnergySlotFloats * hmf::kPostThreads * (int)sizeof(float));
+      if (e != cudaSuccess) return;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, hmf::kPostThreads, pair_smem) != cudaSuccess ||
+          per < 1)
+        per = 1;
+      const long long tiles = (long long)T.tiles_x * T.tiles_y;
+      const long long chunks = std::max<long long>(
+          1, std::min<long long>((2LL * sms * per + tiles - 1) / tiles, (G.vz + 3) / 4));
+      T.zchunk = (int)((G.vz + chunks - 1) / chunks);
+      const long long grid = tiles * ((G.vz + T.zchunk - 1) / T.zchunk);
+      kernel<<<(unsigned)grid, hmf::kPostThreads, pair_smem, s>>>(P, G, T, d_sums);
+    };
     switch (tab.n) {
-      case 1: launch(hmf::energy_reg_kernel<1>); break;
-      case 2: launch(hmf::energy_reg_kernel<2>); break;
-      case 3: launch(hmf::energy_reg_kernel<3>); break;
-      case 4: launch(hmf::energy_reg_kernel<4>); break;
-      case 5: launch(hmf::energy_reg_kernel<5>); break;
-      case 6: launch(hmf::energy_reg_kernel<6>); break;
-      case 7: launch(hmf::energy_reg_kernel<7>); break;
-      default: launch(hmf::energy_reg_kernel<8>); break;
+#define HMF_ENERGY_N(N)                                 \
+  case N:                                                \
+    if (pairs) launch_pairs(hmf::energy_pair_kernel<N>); \
+    else launch(hmf::energy_reg_kernel<N>);              \
+    break;
+      HMF_ENERGY_N(1) HMF_ENERGY_N(2) HMF_ENERGY_N(3) HMF_ENERGY_N(4) HMF_ENERGY_N(5) HMF_ENERGY_N(6)
+      HMF_ENERGY_N(7) HMF_ENERGY_N(8)
+#undef HMF_ENERGY_N
     }
-    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
   } else if (e == cudaSuccess) {
     e = cudaMemcpyAsync(d_tab, &tab, sizeof(tab), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
@@ -114,7 +151,7 @@ int launch_energy(hmf_ctx* c, const hmf::EnergyTable& tab, const hmf::Geometry& 
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(sums.data(), d_sums, sizeof(double) * sums.size(), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (own) cudaFree(own);
+  if (own) pool ? cudaFreeAsync(own, s) : cudaFree(own);
   if (e != cudaSuccess) return cuda_fail(c, e, "energy_kernel");
   if (f0) *f0 = sums[0];
   for (int v = 0; v < n_nodes && f; ++v) f[v] = sums[1 + v];
