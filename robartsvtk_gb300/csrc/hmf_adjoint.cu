@@ -231,9 +231,9 @@ int plan_reverse(hmf_ctx* c, cudaStream_t s) {
   const auto& V = c->vols[0];
   hmf::FlowVolume& F = S->h_avol;
   F.G = c->geo;
-  const int nx = (V.vx + hmf::kAfMaxOut - 1) / hmf::kAfMaxOut;
-  const int ny = (V.vy + hmf::kAfMaxOut - 1) / hmf::kAfMaxOut;
-  F.out_x = (V.vx + nx - 1) / nx;
+  const int nx = (V.vx + hmf::kAfMaxOutX - 1) / hmf::kAfMaxOutX;
+  const int ny = (V.vy + hmf::kAfMaxOutY - 1) / hmf::kAfMaxOutY;
+  F.out_x = ((V.vx + nx - 1) / nx + 1) & ~1;  // even: a thread owns two columns
   F.out_y = (V.vy + ny - 1) / ny;
   F.tiles_x = nx;
   const long long per_chunk = (long long)nx * ny * (c->n - 1);
@@ -498,6 +498,7 @@ int backward_step(hmf_ctx* c, const Staged& staged, int slotA, int slotB, int cu
     hmf::AdjFlowParams fp;
     fp.step = c->step;
     fp.icc = 1.0f / c->cc;
+    fp.neg_zero = -0.0f;
     fp.parity = S->pb_par;
     fp.n_vertices = n - 1;
     fp.vols = S->d_avol;

@@ -8,11 +8,15 @@
 // flows and of the gradient-step values g.  Its stencil chain
 //   g -> p' -> (|p|, m, adjoint of m -> F2b) -> q -> gb -> old-flow adjoint
 // reaches three voxels to the low side and two to the high side, so a CTA
-// owns a 32 x 32 (x, y) window with up to 27 x 27 outputs and marches along
-// z: lane = column x0-3+lane, warp w holds rows 2w and 2w+1 (y0-3+row) in
-// registers; x neighbours move by warp shuffles, y neighbours across a warp
-// boundary through small exchange rows in shared memory, z neighbours stay
-// in registers.  Per plane k the CTA computes g,
+// owns a 32 x 32 (x, y) window with up to 26 x 27 outputs (the window starts
+// four columns low, so that its pairs of columns are 8-byte aligned) and
+// marches along z.  A half-warp covers a row (y0-3+row), two neighbouring
+// columns (x0-4+2 lane) per lane as one 64-bit register pair: loads and stores
+// move 8 bytes and the arithmetic is packed (hmf_f32x2.cuh).  x neighbours are
+// the pair's other half or one warp shuffle, y neighbours go through exchange
+// rows in shared memory, z neighbours stay in registers.  Beyond the high faces
+// p', t and q are zero, so what the reference leaves out there is added as
+// zero.  Per plane k the CTA computes g,
 // p' and the total new-flow adjoint t on plane k, m / F2b and q on k-1, gb on
 // k-2 and the old-flow adjoints on k-3 (two __syncthreads per plane).  Input
 // planes arrive by cp.async.bulk.tensor into mbarrier rings two planes ahead;
@@ -21,11 +25,19 @@
 // warps' first lanes (one array each, one mbarrier arrival per array), and
 // the steady planes of the march -- every stage active, no z boundary near --
 // run a copy of the step compiled without those tests.
+//
+// What bounds it: latency and issue with the 16 warps that its registers and
+// rings allow (54 % of the issue slots, DRAM at 30 %).  128^3, 4 leaves: 198 us a
+// launch, against 211 us with one column and two rows per thread, scalar
+// arithmetic and the alpha gradient's sum in double (138 -> 111 million
+// instructions).
 #pragma once
 
 #include <cuda.h>
 
 #include "hmf_async.cuh"
+#include "hmf_f32x2.cuh"
+#include "hmf_multiplier.cuh"
 #include "hmf_types.cuh"
 
 namespace hmf {
@@ -41,12 +53,12 @@ constexpr int kAfPzSlots = 4;
 // kAfMainSlots and kAfPzSlots - 1.
 constexpr int kAfMainLead = 2;
 constexpr int kAfPzLead = 2;
-constexpr int kAfR = 2;                     // rows per thread
-constexpr int kAfWarps = 32 / kAfR;
-constexpr int kAfThreads = 32 * kAfWarps;   // 512
-constexpr int kAfX = (kAfWarps + 2) * 32;   // exchange row per warp, plus zero rows for warps -1 and 16
+constexpr int kAfRows = 32;                 // window rows, one per half-warp
+constexpr int kAfThreads = 16 * kAfRows;    // 512
+constexpr int kAfWarps = kAfThreads / 32;
+constexpr int kAfX = (kAfRows + 2) * 32;    // one exchange row per window row, plus zero rows -1 and 32
 constexpr int kAfXPlanes = 11;              // g, p'y[2], ty[2], m, F2b, qy[2], dbo[2]
-constexpr int kAfMaxOut = 27;
+constexpr int kAfMaxOutX = 26, kAfMaxOutY = 27;
 constexpr int kAfSmemBytes =
     (kAfMainSlots * kAfMainArrays + kAfPzSlots) * kAfPlane * 4 + kAfXPlanes * kAfX * 4 + 64;
 
@@ -63,6 +75,7 @@ struct AdjFlowVertex {  // 64-byte aligned through its CUtensorMap members
 
 struct AdjFlowParams {
   float step, icc;
+  float neg_zero;  // -0: the addend of packed multiplications (hmf_f32x2.cuh)
   int parity;      // which Pb set is read (the other is written)
   int n_vertices;  // grid.x = n_vertices * items
   const FlowVolume* vols;
@@ -71,17 +84,28 @@ struct AdjFlowParams {
   unsigned long long wait_limit_ns;  // bound of every copy wait (kTmaWaitLimitNs unless a caller sets it)
 };
 
+// Float-float running sum: each term is added with Knuth's TwoSum, its rounding
+// error collected in lo.
+struct FF {
+  float hi, lo;
+};
+__device__ __forceinline__ void ff_accumulate(FF& a, float t) {
+  const float s = a.hi + t, b = s - a.hi;
+  a.lo += (a.hi - (s - b)) + (t - b);
+  a.hi = s;
+}
+
 __global__ void __launch_bounds__(kAfThreads, 1)
 adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowParams fp) {
   extern __shared__ __align__(1024) unsigned char af_raw[];
   float* mslots = reinterpret_cast<float*>(af_raw);                      // [3][10][1216]
   float* zslots = mslots + kAfMainSlots * kAfMainArrays * kAfPlane;      // [4][1216]
-  float* xp = zslots + kAfPzSlots * kAfPlane;                            // [11][18][32]
+  float* xp = zslots + kAfPzSlots * kAfPlane;                            // [11][34][32]
   uint64_t* mbars = reinterpret_cast<uint64_t*>(xp + kAfXPlanes * kAfX); // [3]
   uint64_t* zbars = mbars + kAfMainSlots;                                // [4]
   uint64_t* stall_bar = zbars + kAfPzSlots;                              // [1] never completed (a requested stall)
-  // exchange rows: *_L = the last row of each warp (read by the next warp as
-  // its y-1 neighbour), *_F = the first row (read by the previous warp as y+1)
+  // exchange rows: *_L is read by the row above it (its y-1 neighbour), *_F by
+  // the row below (y+1)
   float* XG_L = xp;
   float* XPPY_F = xp + 1 * kAfX;  // [2] by plane parity
   float* XTY_F = xp + 3 * kAfX;   // [2]
@@ -103,9 +127,10 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
   const int ocols = FV.out_x, orows = FV.out_y;
   const int x0 = (item.tile % FV.tiles_x) * ocols;
   const int y0 = (item.tile / FV.tiles_x) * orows;
-  const int xs = ((x0 + 1) / 4) * 4 - 4;  // x0 - 3 rounded down to a multiple of 4 (x0 >= 0)
-  const int off = (x0 - 3) - xs;           // 0..3
-  const int x = x0 - 3 + lane;
+  const int xs = (x0 / 4) * 4 - 4;        // x0 - 4 rounded down to a multiple of 4 (x0 >= 0, even)
+  const int off = (x0 - 4) - xs;           // 0 or 2
+  const int col = (lane & 15) * 2, row = warp * 2 + (lane >> 4);
+  const int x = x0 - 4 + col, y = y0 - 3 + row;
   const int zs = item.zc * FV.zchunk;
   const int ze = min(zs + FV.zchunk, G.vz);
   const int kstart = max(zs - 3, 0);
@@ -121,23 +146,20 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
   float* const oy = V->pb_out[par][1];
   float* const oz = V->pb_out[par][2];
   float* const ogb = V->gb;
-  const bool xin = x >= 0 && x < G.vx, xpos = x > 0, xnl = x != G.vx - 1;
-  const bool xown = xin && lane >= 3 && lane < 3 + ocols;
-  bool rin[kAfR], ypos[kAfR], ynl[kAfR], rown[kAfR];
-  long long rowoff[kAfR];
-  int si[kAfR];
+  const bool yin = y >= 0 && y < G.vy;
+  bool in[2], face_x[2], face_y[2];  // the pair's voxels inside the volume; and off its low x / y face
 #pragma unroll
-  for (int j = 0; j < kAfR; ++j) {
-    const int row = warp * kAfR + j;
-    const int y = y0 - 3 + row;
-    rin[j] = xin && y >= 0 && y < G.vy;
-    ypos[j] = y > 0;
-    ynl[j] = y != G.vy - 1;
-    rown[j] = rin[j] && xown && row >= 3 && row < 3 + orows;
-    rowoff[j] = (long long)y * G.pitch + x;
-    si[j] = row * kAfBoxX + off + lane;  // element in a staged plane
+  for (int j = 0; j < 2; ++j) {
+    in[j] = yin && x + j >= 0 && x + j < G.vx;
+    face_x[j] = in[j] && x + j > 0;
+    face_y[j] = in[j] && y > 0;
   }
-  const int xw = (warp + 1) * 32 + lane;  // this warp's entry in an exchange row
+  // outputs: pairs of columns (ocols is even; the second may be the first
+  // padding column, which gets zero)
+  const bool own = in[0] && col >= 4 && col < 4 + ocols && row >= 3 && row < 3 + orows;
+  const long long rowoff = (long long)y * G.pitch + x;
+  const int si = row * kAfBoxX + off + col;  // element in a staged plane
+  const int xw = (row + 1) * 32 + col;       // this pair's entry in an exchange row
 
   if (threadIdx.x == 0) {
     const int flag = fp.error_flag ? *(volatile int*)fp.error_flag : 0;
@@ -154,7 +176,7 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     stop = 0;
   }
-  // exchange rows of warps -1 and 16 are read as zeros (never written)
+  // exchange rows -1 and 32 are read as zeros (never written)
   for (int i = threadIdx.x; i < kAfXPlanes * kAfX; i += kAfThreads) xp[i] = 0.f;
   __syncthreads();
   if (abort_cta) return;
@@ -213,29 +235,30 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
   }
   __syncthreads();
 
-  // A window whose 32 x 32 columns / rows lie strictly inside the volume (not
-  // on its first or last column / row) needs none of the x / y boundary
-  // masks; it runs a copy of the march with them folded away.
-  const bool interior = x0 - 3 >= 1 && x0 + 28 <= G.vx - 2 && y0 - 3 >= 1 && y0 + 28 <= G.vy - 2;
-  double asum = 0.0;
+  // A window whose 32 x 32 columns / rows lie inside the volume and off its low
+  // faces needs none of the x / y boundary masks; it runs a copy of the march
+  // with them folded away.
+  const bool interior = x0 - 4 >= 1 && x0 + 27 <= G.vx - 1 && y0 - 3 >= 1 && y0 + 28 <= G.vy - 1;
+  FF asum{0.0f, 0.0f};  // alpha gradient (float-float: this part's FP64 rate is 1/64 of its FP32 rate)
 
   auto march = [&](auto tag) {
     constexpr bool INT = decltype(tag)::value;
-    const bool vxpos = INT || xpos, vxnl = INT || xnl;
-    // carries, one per row of this thread
-    float gprev[kAfR], dbp_prev[kAfR];                                        // plane k-1
-    float ppx_c[kAfR], ppy_c[kAfR], ppz_c[kAfR], tx_c[kAfR], ty_c[kAfR], tz_c[kAfR], S_c[kAfR];  // k-1
-    float m_prev[kAfR], f_prev[kAfR];                                         // plane k-2
-    float qx_e[kAfR], qy_e[kAfR], qz_e[kAfR];                                 // q of plane k-2
-    float qx_f[kAfR], qy_f[kAfR], qz_f[kAfR];                                 // q of plane k-3
-    float dbo_f[kAfR], dbo_ff[kAfR];                                          // dbo of planes k-3, k-4
-    float pzn_c[kAfR];
-#pragma unroll
-    for (int j = 0; j < kAfR; ++j) {
-      gprev[j] = dbp_prev[j] = ppx_c[j] = ppy_c[j] = ppz_c[j] = tx_c[j] = ty_c[j] = tz_c[j] = S_c[j] = 0.f;
-      m_prev[j] = 1.f;
-      f_prev[j] = qx_e[j] = qy_e[j] = qz_e[j] = qx_f[j] = qy_f[j] = qz_f[j] = dbo_f[j] = dbo_ff[j] = pzn_c[j] = 0.f;
-    }
+    const F2 zero2 = f2(0.f), half2 = f2(0.5f), two2 = f2(2.0f), step2 = f2(step), icc2 = f2(icc), alpha2 = f2(alpha);
+    const F2 nz2 = f2(fp.neg_zero);
+    auto mul = [&](F2 a, F2 b) { return f2_mul(a, b, nz2); };
+    auto left = [&](F2 a) { return f2(__shfl_up_sync(FULL, f2_hi(a), 1, 16), f2_lo(a)); };      // at x - 1
+    auto right = [&](F2 a) { return f2(f2_hi(a), __shfl_down_sync(FULL, f2_lo(a), 1, 16)); };  // at x + 1
+    auto inside = [&](F2 a) { return INT ? a : f2_mask(a, in[0], in[1]); };
+    auto off_x = [&](F2 a) { return INT ? a : f2_mask(a, face_x[0], face_x[1]); };
+    auto off_y = [&](F2 a) { return INT ? a : f2_mask(a, face_y[0], face_y[1]); };
+    // carries
+    F2 gprev = zero2, dbp_prev = zero2;                                                              // plane k-1
+    F2 ppx = zero2, ppy = zero2, ppz = zero2, tx = zero2, ty = zero2, tz = zero2, S_c = zero2;       // k-1
+    F2 m_prev = f2(1.0f), f_prev = zero2;                                                            // k-2
+    F2 qx_e = zero2, qy_e = zero2, qz_e = zero2;                                                     // q of k-2
+    F2 qx_f = zero2, qy_f = zero2, qz_f = zero2;                                                     // q of k-3
+    F2 dbo_f = zero2, dbo_ff = zero2;                                                                // k-3, k-4
+    F2 pzn_c = zero2;
     bool have_pz = false;
     const float* cur = mslot(kstart);
     const float* zc = zslot(kstart);
@@ -256,43 +279,36 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
       const int kb = k & 1;  // exchange-row parity of plane k
 
       // ---- stage A: g(k) (kern_CalcGradStep on the recomputed divergence)
-      float g[kAfR], px[kAfR], py[kAfR], pz[kAfR], Pbx[kAfR], Pby[kAfR], Pbz[kAfR], dbp[kAfR], dbpl[kAfR],
-          dbpu[kAfR], Sk[kAfR];
-#pragma unroll
-      for (int j = 0; j < kAfR; ++j)
-        g[j] = px[j] = py[j] = pz[j] = Pbx[j] = Pby[j] = Pbz[j] = dbp[j] = dbpl[j] = dbpu[j] = Sk[j] = 0.f;
+      F2 g = zero2, px = zero2, py = zero2, pz = zero2, Pbx = zero2, Pby = zero2, Pbz = zero2, dbp = zero2,
+         dbpl = zero2, dbpu = zero2, Sk = zero2;
       if (doA) {
         const bool has_next = ST || k + 1 < G.vz;
         const int znext = zsi + 1 == kAfPzSlots ? 0 : zsi + 1;
         const float* zn = zslots + znext * kAfPlane;
-#pragma unroll
-        for (int j = 0; j < kAfR; ++j) {
-          const int e = si[j];
-          px[j] = cur[e];
-          py[j] = cur[kAfPlane + e];
-          pz[j] = (ST || have_pz) ? pzn_c[j] : zc[e];
-          const float pxr = cur[e + 1];
-          const float pyd = cur[kAfPlane + e + kAfBoxX];
-          const float pzn = has_next ? zn[e] : 0.f;
-          const float sk = cur[2 * kAfPlane + e], c = cur[3 * kAfPlane + e], u = cur[4 * kAfPlane + e];
-          Pbx[j] = cur[5 * kAfPlane + e];
-          Pby[j] = cur[6 * kAfPlane + e];
-          Pbz[j] = cur[7 * kAfPlane + e];
-          dbp[j] = cur[8 * kAfPlane + e];
-          dbpl[j] = (off + lane) > 0 ? cur[8 * kAfPlane + e - 1] : 0.f;
-          dbpu[j] = (warp * kAfR + j) > 0 ? cur[8 * kAfPlane + e - kAfBoxX] : 0.f;
-          Sk[j] = has_s ? cur[9 * kAfPlane + e] : 0.f;
-          float d = (px[j] + py[j]) + pz[j];
-          if (vxnl) d = d - pxr;
-          if (INT || ynl[j]) d = d - pyd;
-          if (has_next) d = d - pzn;
-          const float gv = step * (((sk + d) - c) - u * icc);
-          g[j] = (INT || rin[j]) ? gv : 0.f;
-          pzn_c[j] = pzn;
-        }
+        px = f2_ld(cur + si);
+        py = f2_ld(cur + kAfPlane + si);
+        pz = (ST || have_pz) ? pzn_c : f2_ld(zc + si);
+        const F2 pxr = f2(f2_hi(px), cur[si + 2]);
+        const F2 pyd = f2_ld(cur + kAfPlane + si + kAfBoxX);
+        const F2 pzn = has_next ? f2_ld(zn + si) : zero2;
+        const F2 sk = f2_ld(cur + 2 * kAfPlane + si), c = f2_ld(cur + 3 * kAfPlane + si),
+                 u = f2_ld(cur + 4 * kAfPlane + si);
+        Pbx = f2_ld(cur + 5 * kAfPlane + si);
+        Pby = f2_ld(cur + 6 * kAfPlane + si);
+        Pbz = f2_ld(cur + 7 * kAfPlane + si);
+        dbp = f2_ld(cur + 8 * kAfPlane + si);
+        dbpl = f2(off + col > 0 ? cur[8 * kAfPlane + si - 1] : 0.f, f2_lo(dbp));
+        dbpu = row > 0 ? f2_ld(cur + 8 * kAfPlane + si - kAfBoxX) : zero2;
+        if (has_s) Sk = f2_ld(cur + 9 * kAfPlane + si);
+        F2 d = (px + py) + pz;
+        d = d - pxr;
+        d = d - pyd;
+        d = d - pzn;
+        g = mul(step2, ((sk + d) - c) - mul(u, icc2));
+        pzn_c = pzn;
         have_pz = has_next;
       }
-      XG_L[xw] = g[kAfR - 1];
+      f2_st(XG_L + xw, g);
       __syncthreads();  // (1)
       if (lane == 0) {
         if (warp < narr && k + kAfMainLead <= kA_end) issue_main_array(k + kAfMainLead, warp, warp_map);
@@ -301,76 +317,72 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
 
       // ---- stage B: p'(k) (kern_DescentSpatialFlow) and the total adjoint t(k)
       // of the new flows (incoming plus through the new divergence)
-      float ppx_n[kAfR], ppy_n[kAfR], ppz_n[kAfR], tx_n[kAfR], ty_n[kAfR], tz_n[kAfR];
-      {
-        const float gup = XG_L[xw - 32];
-#pragma unroll
-        for (int j = 0; j < kAfR; ++j) {
-          const float gxm = __shfl_up_sync(FULL, g[j], 1);
-          const float gym = j ? g[j > 0 ? j - 1 : 0] : gup;
-          const bool vin = doA && (INT || rin[j]);
-          const bool vyp = INT || ypos[j];
-          ppx_n[j] = (vin && vxpos) ? px[j] - (g[j] - gxm) : 0.f;
-          ppy_n[j] = (vin && vyp) ? py[j] - (g[j] - gym) : 0.f;
-          ppz_n[j] = (vin && (ST || k > 0)) ? pz[j] - (g[j] - gprev[j]) : 0.f;
-          tx_n[j] = vin ? (Pbx[j] + dbp[j]) - (vxpos ? dbpl[j] : 0.f) : 0.f;
-          ty_n[j] = vin ? (Pby[j] + dbp[j]) - (vyp ? dbpu[j] : 0.f) : 0.f;
-          tz_n[j] = vin ? (Pbz[j] + dbp[j]) - ((ST || k > 0) ? dbp_prev[j] : 0.f) : 0.f;
-          if (doA) {
-            gprev[j] = g[j];
-            dbp_prev[j] = dbp[j];
-          }
-        }
-        XPPY_F[kb * kAfX + xw] = ppy_n[0];
-        XTY_F[kb * kAfX + xw] = ty_n[0];
+      F2 ppx_n = off_x(px - (g - left(g)));
+      F2 ppy_n = off_y(py - (g - f2_ld(XG_L + xw - 32)));
+      F2 ppz_n = inside(pz - (g - gprev));
+      F2 tx_n = inside((Pbx + dbp) - dbpl);
+      F2 ty_n = inside((Pby + dbp) - dbpu);
+      F2 tz_n = inside((Pbz + dbp) - ((ST || k > 0) ? dbp_prev : zero2));
+      if (!ST) {
+        if (!doA) ppx_n = ppy_n = ppz_n = tx_n = ty_n = tz_n = zero2;
+        if (k <= 0) ppz_n = zero2;
       }
+      if (doA) {
+        gprev = g;
+        dbp_prev = dbp;
+      }
+      f2_st(XPPY_F + kb * kAfX + xw, ppy_n);
+      f2_st(XTY_F + kb * kAfX + xw, ty_n);
 
       // ---- stage C: |p|, m(k-1) and the adjoint of the multiplier -> F2b(k-1)
-      float m[kAfR], f2b[kAfR];
+      F2 m = f2(1.0f), f2b = zero2;
       {
-        const float pdown = XPPY_F[(kb ^ 1) * kAfX + xw + 32];
-        const float tdown = XTY_F[(kb ^ 1) * kAfX + xw + 32];
-        const bool znl = ST || kc != G.vz - 1;
+        const F2 pyd = f2_ld(XPPY_F + (kb ^ 1) * kAfX + xw + 32);
+        const F2 tyd = f2_ld(XTY_F + (kb ^ 1) * kAfX + xw + 32);
+        const F2 pxr = right(ppx), txr = right(tx);
+        F2 f = mul(ppx, ppx) + mul(pxr, pxr);
+        f = f + (mul(ppy, ppy) + mul(pyd, pyd));
+        f = f + (mul(ppz, ppz) + mul(ppz_n, ppz_n));
+        const F2 h = mul(half2, f);
+        const F2 lim = has_s ? mul(alpha2, S_c) : alpha2;
+        // above 1e-36: |p| <= lim exactly and m = 1 (as in flow_tma_kernel)
+        F2 slack = mul(mul(lim, lim), f2(1.0f - 0x1p-20f)) - h;
+        if (!INT) slack = f2(in[0] ? f2_lo(slack) : 1.0f, in[1] ? f2_hi(slack) : 1.0f);
+        const bool near0 = doC && !(f2_lo(slack) > 1.0e-36f), near1 = doC && !(f2_hi(slack) > 1.0e-36f);
+        if (__any_sync(FULL, near0 || near1)) {
+          F2 mb2 = mul(mul(tx, half2), ppx);  // (terms of the reference's masked faces are zero: p' is)
+          mb2 = zero2 + mb2;
+          mb2 = mb2 + mul(mul(txr, half2), pxr);
+          mb2 = mb2 + mul(mul(ty, half2), ppy);
+          mb2 = mb2 + mul(mul(tyd, half2), pyd);
+          mb2 = mb2 + mul(mul(tz, half2), ppz);
+          mb2 = mb2 + mul(mul(tz_n, half2), ppz_n);
+          float mv[2] = {1.0f, 1.0f}, fv[2] = {0.0f, 0.0f};
 #pragma unroll
-        for (int j = 0; j < kAfR; ++j) {
-          const float pxr = __shfl_down_sync(FULL, ppx_c[j], 1);
-          const float txr = __shfl_down_sync(FULL, tx_c[j], 1);
-          const float pyd = j < kAfR - 1 ? ppy_c[j < kAfR - 1 ? j + 1 : j] : pdown;
-          const float tyd = j < kAfR - 1 ? ty_c[j < kAfR - 1 ? j + 1 : j] : tdown;
-          m[j] = 1.f;
-          f2b[j] = 0.f;
-          if (doC && (INT || rin[j])) {
-            const bool vyp = INT || ypos[j], vyn = INT || ynl[j];
-            float up = ppx_c[j] * ppx_c[j];
-            float dn = vxnl ? pxr * pxr : 0.f;
-            float F = up + dn;
-            up = ppy_c[j] * ppy_c[j];
-            dn = vyn ? pyd * pyd : 0.f;
-            F = F + (up + dn);
-            up = ppz_c[j] * ppz_c[j];
-            dn = znl ? ppz_n[j] * ppz_n[j] : 0.f;
-            F = F + (up + dn);
-            const float h = 0.5f * F;
-            const float lim = has_s ? alpha * S_c[j] : alpha;
-            if (!(lim > 1.0e-18f && h < (lim * lim) * (1.0f - 0x1p-20f))) {  // else |p| <= lim exactly: m = 1
-              const float Fm = sqrtf(h);
-              if (Fm > lim) {
-                float mb = 0.f;
-                if (vxpos) mb = mb + (tx_c[j] * 0.5f) * ppx_c[j];
-                if (vxnl) mb = mb + (txr * 0.5f) * pxr;
-                if (vyp) mb = mb + (ty_c[j] * 0.5f) * ppy_c[j];
-                if (vyn) mb = mb + (tyd * 0.5f) * pyd;
-                if (ST || kc > 0) mb = mb + (tz_c[j] * 0.5f) * ppz_c[j];
-                if (znl) mb = mb + (tz_n[j] * 0.5f) * ppz_n[j];
-                m[j] = lim / Fm;
-                f2b[j] = -mb * lim / (4.0f * Fm * Fm * Fm);
-                if (rown[j] && (ST || kc >= zs) && kc < ze) asum += (double)(mb / Fm * (has_s ? S_c[j] : 1.0f));
+          for (int j = 0; j < 2; ++j) {
+            const float hj = j ? f2_hi(h) : f2_lo(h), lj = j ? f2_hi(lim) : f2_lo(lim);
+            if (j ? near1 : near0) {
+              float Fm, mj;
+              if (multiplier_unsafe(hj, lj)) {
+                Fm = sqrtf(hj);
+                mj = lj / Fm;
+              } else {
+                mj = multiplier_root(hj, lj, Fm);
+              }
+              if (Fm > lj) {
+                const float mb = j ? f2_hi(mb2) : f2_lo(mb2);
+                mv[j] = mj;
+                fv[j] = -mb * lj / (4.0f * Fm * Fm * Fm);
+                if (own && (j == 0 || in[1]) && (ST || kc >= zs) && kc < ze)
+                  ff_accumulate(asum, mb / Fm * (has_s ? (j ? f2_hi(S_c) : f2_lo(S_c)) : 1.0f));
               }
             }
           }
+          m = f2(mv[0], mv[1]);
+          f2b = f2(fv[0], fv[1]);
         }
-        XM_L[xw] = m[kAfR - 1];
-        XF_L[xw] = f2b[kAfR - 1];
+        f2_st(XM_L + xw, m);
+        f2_st(XF_L + xw, f2b);
       }
       if (threadIdx.x == 0) {  // the planes the next step's stage A reads
         if (k + 1 <= kA_end) wait_main0(k + 1);
@@ -383,86 +395,61 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
       }
 
       // ---- stage D: q(k-1), the adjoint of p'
-      float qx_n[kAfR], qy_n[kAfR], qz_n[kAfR];
-      {
-        const float mup = XM_L[xw - 32], fup = XF_L[xw - 32];
-#pragma unroll
-        for (int j = 0; j < kAfR; ++j) {
-          const float mxm = __shfl_up_sync(FULL, m[j], 1);
-          const float fxm = __shfl_up_sync(FULL, f2b[j], 1);
-          const float mym = j ? m[j > 0 ? j - 1 : 0] : mup;
-          const float fym = j ? f2b[j > 0 ? j - 1 : 0] : fup;
-          qx_n[j] = qy_n[j] = qz_n[j] = 0.f;
-          if (doC && (INT || rin[j])) {
-            qx_n[j] = vxpos ? (tx_c[j] * 0.5f) * (m[j] + mxm) + (2.0f * ppx_c[j]) * (f2b[j] + fxm) : 0.f;
-            qy_n[j] = (INT || ypos[j]) ? (ty_c[j] * 0.5f) * (m[j] + mym) + (2.0f * ppy_c[j]) * (f2b[j] + fym) : 0.f;
-            qz_n[j] = (ST || kc > 0) ? (tz_c[j] * 0.5f) * (m[j] + m_prev[j]) + (2.0f * ppz_c[j]) * (f2b[j] + f_prev[j])
-                                      : 0.f;
-          }
-          if (doC) {
-            m_prev[j] = m[j];
-            f_prev[j] = f2b[j];
-          }
-        }
-        XQY_F[(kb ^ 1) * kAfX + xw] = qy_n[0];  // plane k-1
+      F2 qx_n = zero2, qy_n = zero2, qz_n = zero2;
+      if (doC) {
+        const F2 mup = f2_ld(XM_L + xw - 32), fup = f2_ld(XF_L + xw - 32);
+        qx_n = off_x(mul(mul(tx, half2), m + left(m)) + mul(mul(two2, ppx), f2b + left(f2b)));
+        qy_n = off_y(mul(mul(ty, half2), m + mup) + mul(mul(two2, ppy), f2b + fup));
+        if (ST || kc > 0) qz_n = inside(mul(mul(tz, half2), m + m_prev) + mul(mul(two2, ppz), f2b + f_prev));
+        m_prev = m;
+        f_prev = f2b;
       }
+      f2_st(XQY_F + (kb ^ 1) * kAfX + xw, qy_n);  // plane k-1
 
       // ---- stage E: gb(k-2), the adjoint of g, and dbo = step * gb
-      float dbo[kAfR];
+      F2 dbo = zero2;
       {
-        const float qdown = XQY_F[kb * kAfX + xw + 32];  // plane k-2
-#pragma unroll
-        for (int j = 0; j < kAfR; ++j) {
-          const float qxr = __shfl_down_sync(FULL, qx_e[j], 1);
-          const float qyd = j < kAfR - 1 ? qy_e[j < kAfR - 1 ? j + 1 : j] : qdown;
-          dbo[j] = 0.f;
-          if (doE && (INT || rin[j])) {
-            float gb = -((qx_e[j] + qy_e[j]) + qz_e[j]);
-            if (vxnl) gb = gb + qxr;
-            if (INT || ynl[j]) gb = gb + qyd;
-            if (ST || ko != G.vz - 1) gb = gb + qz_n[j];
-            dbo[j] = step * gb;
-            if (rown[j] && (ST || ko >= zs)) ogb[go + rowoff[j]] = gb;
-          }
+        const F2 qyd = f2_ld(XQY_F + kb * kAfX + xw + 32);  // plane k-2
+        const F2 s3 = (qx_e + qy_e) + qz_e;
+        F2 gb = f2(-f2_lo(s3), -f2_hi(s3));
+        gb = gb + right(qx_e);
+        gb = gb + qyd;
+        gb = gb + qz_n;
+        if (doE) {
+          dbo = inside(mul(step2, gb));
+          if (own && (ST || ko >= zs)) f2_st(ogb + (go + rowoff), inside(gb));
         }
-        XD_L[kb * kAfX + xw] = dbo[kAfR - 1];  // plane k-2
+        f2_st(XD_L + kb * kAfX + xw, dbo);  // plane k-2
       }
 
       // ---- stage F: adjoint of the old flows at k-3
       {
-        const float dup = XD_L[(kb ^ 1) * kAfX + xw - 32];  // plane k-3
-#pragma unroll
-        for (int j = 0; j < kAfR; ++j) {
-          const float dxl = __shfl_up_sync(FULL, dbo_f[j], 1);
-          const float dyu = j ? dbo_f[j > 0 ? j - 1 : 0] : dup;
-          if (doF && rown[j]) {
-            const long long o = fo + rowoff[j];
-            ox[o] = (qx_f[j] + dbo_f[j]) - (vxpos ? dxl : 0.f);
-            oy[o] = (qy_f[j] + dbo_f[j]) - ((INT || ypos[j]) ? dyu : 0.f);
-            oz[o] = (qz_f[j] + dbo_f[j]) - ((ST || kf > 0) ? dbo_ff[j] : 0.f);
-          }
+        const F2 dup = f2_ld(XD_L + (kb ^ 1) * kAfX + xw - 32);  // plane k-3
+        const F2 dxl = left(dbo_f);
+        if (doF && own) {
+          const long long o = fo + rowoff;
+          f2_st(ox + o, inside((qx_f + dbo_f) - dxl));
+          f2_st(oy + o, inside((qy_f + dbo_f) - dup));
+          f2_st(oz + o, inside((qz_f + dbo_f) - ((ST || kf > 0) ? dbo_ff : zero2)));
         }
       }
 
       // ---- rotate carries and ring positions
-#pragma unroll
-      for (int j = 0; j < kAfR; ++j) {
-        ppx_c[j] = ppx_n[j];
-        ppy_c[j] = ppy_n[j];
-        ppz_c[j] = ppz_n[j];
-        tx_c[j] = tx_n[j];
-        ty_c[j] = ty_n[j];
-        tz_c[j] = tz_n[j];
-        S_c[j] = Sk[j];
-        qx_f[j] = qx_e[j];
-        qy_f[j] = qy_e[j];
-        qz_f[j] = qz_e[j];
-        qx_e[j] = qx_n[j];
-        qy_e[j] = qy_n[j];
-        qz_e[j] = qz_n[j];
-        dbo_ff[j] = dbo_f[j];
-        dbo_f[j] = dbo[j];
-      }
+      ppx = ppx_n;
+      ppy = ppy_n;
+      ppz = ppz_n;
+      tx = tx_n;
+      ty = ty_n;
+      tz = tz_n;
+      S_c = Sk;
+      qx_f = qx_e;
+      qy_f = qy_e;
+      qz_f = qz_e;
+      qx_e = qx_n;
+      qy_e = qy_n;
+      qz_e = qz_n;
+      dbo_ff = dbo_f;
+      dbo_f = dbo;
       msi = msi + 1 == kAfMainSlots ? 0 : msi + 1;
       zsi = zsi + 1 == kAfPzSlots ? 0 : zsi + 1;
       cur = mslots + msi * (kAfMainArrays * kAfPlane);
@@ -483,8 +470,9 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
   const bool timed_out = stop != 0;
 
   // alpha gradient: block sum, one atomic per CTA
-  for (int o = 16; o > 0; o >>= 1) asum += __shfl_down_sync(FULL, asum, o);
-  if (lane == 0) red[warp] = asum;
+  double alpha_sum = (double)asum.hi + (double)asum.lo;
+  for (int o = 16; o > 0; o >>= 1) alpha_sum += __shfl_down_sync(FULL, alpha_sum, o);
+  if (lane == 0) red[warp] = alpha_sum;
   __syncthreads();
   if (warp == 0) {
     double v = lane < kAfWarps ? red[lane] : 0.0;
