@@ -260,8 +260,10 @@ int hmf_get_flow_units(const hmf_ctx* ctx);
  * are cut at the flow plan's z chunks into per-slab graph nodes that wait
  * only for the slabs their stencil touches, so sweeps overlap flows and
  * consecutive iterations overlap.  Same arithmetic, bit-identical results.
- * On by default; hmf_get_pipeline returns 1 when the next solve runs
- * pipelined. */
+ * On by default; hmf_get_pipeline returns 1 when it is on and the plan allows
+ * it.  On the default plan a volume small enough for the whole flow step to be
+ * resident at once runs in whole launches all the same (a z chunk, window or
+ * units per CTA set by the caller are pipelined at any size). */
 int hmf_set_pipeline(hmf_ctx* ctx, int enabled);
 int hmf_get_pipeline(const hmf_ctx* ctx);
 

@@ -383,8 +383,10 @@ int build_transition_tables(hmf_ctx* c, const Staged& staged, cudaStream_t s) {
 // one forward iteration with the tables of pair `pair`
 int forward_iteration(hmf_ctx* c, int pair, cudaStream_t s) {
   AdjointState* S = c->adj;
+  c->overlap_launches = true;
   int rc = launch_flow_tma_with(c, S->d_tflow + (size_t)pair * (c->n - 1), 0, s);
   if (!rc) rc = launch_tree_bulk_with(c, S->d_ttree + pair, s);
+  c->overlap_launches = false;
   return rc;
 }
 
@@ -476,22 +478,20 @@ int backward_step(hmf_ctx* c, const Staged& staged, int slotA, int slotB, int cu
     bool flat = c->root == 0;  // every other vertex a leaf of root 0: parents known at compile time
     for (int v = 1; v < n; ++v) flat = flat && c->parent[v] == 0;
     if (int rc = maybe_request_stall(c, HMF_STALL_REVERSE_SWEEP, s)) return rc;
+    auto launch = [&](auto kernel) {
+      return hmf::launch_waiting(true, kernel, dim3(grid), hmf::kSwVc, smem, s, S->d_tree, G, W, c->d_error);
+    };
+    cudaError_t e = cudaErrorInvalidValue;
     switch (n * 4 + (flat ? 2 : pre ? 1 : 0)) {
-#define HMF_SWEEP_CASE(N)                                                                                  \
-  case 4 * N:                                                                                              \
-    hmf::adj_sweep_kernel<N, false, false><<<grid, hmf::kSwVc, smem, s>>>(S->d_tree, G, W, c->d_error);    \
-    break;                                                                                                 \
-  case 4 * N + 1:                                                                                          \
-    hmf::adj_sweep_kernel<N, true, false><<<grid, hmf::kSwVc, smem, s>>>(S->d_tree, G, W, c->d_error);     \
-    break;                                                                                                 \
-  case 4 * N + 2:                                                                                          \
-    hmf::adj_sweep_kernel<N, true, true><<<grid, hmf::kSwVc, smem, s>>>(S->d_tree, G, W, c->d_error);      \
-    break;
+#define HMF_SWEEP_CASE(N)                                             \
+  case 4 * N: e = launch(hmf::adj_sweep_kernel<N, false, false>); break;     \
+  case 4 * N + 1: e = launch(hmf::adj_sweep_kernel<N, true, false>); break;  \
+  case 4 * N + 2: e = launch(hmf::adj_sweep_kernel<N, true, true>); break;
       HMF_SWEEP_CASE(2) HMF_SWEEP_CASE(3) HMF_SWEEP_CASE(4) HMF_SWEEP_CASE(5)
       HMF_SWEEP_CASE(6) HMF_SWEEP_CASE(7) HMF_SWEEP_CASE(8)
 #undef HMF_SWEEP_CASE
     }
-    CK(cudaGetLastError(), "adj_sweep_kernel launch");
+    CK(e, "adj_sweep_kernel launch");
   }
   ++c->launches;
   if (!S->chain) {
@@ -507,9 +507,9 @@ int backward_step(hmf_ctx* c, const Staged& staged, int slotA, int slotB, int cu
     fp.wait_limit_ns = c->wait_limit_ns;
     if (int rc = maybe_request_stall(c, HMF_STALL_REVERSE_FLOW, s)) return rc;
     const dim3 grid((unsigned)S->n_aitems * (unsigned)(n - 1));
-    hmf::adj_flow_tma_kernel<<<grid, hmf::kAfThreads, hmf::kAfSmemBytes, s>>>(
-        S->d_aflow + (size_t)slotA * (n - 1), fp);
-    CK(cudaGetLastError(), "adj_flow_tma_kernel launch");
+    CK(hmf::launch_waiting(true, hmf::adj_flow_tma_kernel, grid, hmf::kAfThreads, hmf::kAfSmemBytes, s,
+                           S->d_aflow + (size_t)slotA * (n - 1), fp),
+       "adj_flow_tma_kernel launch");
     ++c->launches;
     S->pb_par ^= 1;
     return HMF_OK;

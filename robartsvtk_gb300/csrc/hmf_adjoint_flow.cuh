@@ -116,6 +116,7 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
   __shared__ int abort_cta, stall_cta;
   __shared__ int stop;
   __shared__ double red[kAfWarps];
+  dependents_may_launch();
 
   const int nv = fp.n_vertices;
   const FlowItem item = fp.items[blockIdx.x / nv];
@@ -161,6 +162,7 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
   const int si = row * kAfBoxX + off + col;  // element in a staged plane
   const int xw = (row + 1) * 32 + col;       // this pair's entry in an exchange row
 
+  wait_for_previous_grid();
   if (threadIdx.x == 0) {
     const int flag = fp.error_flag ? *(volatile int*)fp.error_flag : 0;
     abort_cta = flag & 2;

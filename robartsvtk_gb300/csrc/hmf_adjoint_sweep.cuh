@@ -62,8 +62,10 @@ __global__ void __launch_bounds__(kSwVc) adj_sweep_kernel(const AdjTree* __restr
   float* stage0 = reinterpret_cast<float*>(sw_raw + 128);
   constexpr int kStage = kSwKinds * N * kSwVc;  // floats per stage
 
+  dependents_may_launch();
   for (int i = threadIdx.x; i < (int)(sizeof(AdjTree) / 4); i += blockDim.x)
     reinterpret_cast<int*>(&T)[i] = reinterpret_cast<const int*>(table)[i];
+  wait_for_previous_grid();
   if (threadIdx.x == 0) {
     const int flag = error_flag ? *(volatile int*)error_flag : 0;
     abort_cta = flag & 2;

@@ -3,9 +3,35 @@
 #pragma once
 
 #include <cuda.h>
+#include <cuda_runtime.h>
 #include <stdint.h>
 
 namespace hmf {
+
+// Programmatic dependent launch: the next kernel of the stream may start once
+// every CTA of this one has said so, and waits, before it touches this one's
+// results, until this one has ended and its writes are visible.  Both do
+// nothing in a kernel launched without the attribute.
+__device__ __forceinline__ void dependents_may_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launches a kernel that waits for the previous one itself: with `overlap` it
+// carries the attribute, without it is an ordinary launch.
+template <class... Params, class... Args>
+cudaError_t launch_waiting(bool overlap, void (*kernel)(Params...), dim3 grid, int threads, size_t smem,
+                           cudaStream_t s, Args... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));

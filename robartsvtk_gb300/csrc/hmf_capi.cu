@@ -282,6 +282,9 @@ int allocate_state(hmf_ctx* c) {
 }
 
 // Output rows of one flow window of the context's shape.
+// Flow CTAs resident at once.
+long long flow_slots(const hmf_ctx* c) { return std::max(1, c->sm_count) * (c->flow_warps <= 8 ? 2LL : 1LL); }
+
 int flow_max_out_y(const hmf_ctx* c) { return 4 * c->flow_warps - 5; }
 
 // Flow-kernel work plan for a given z-chunk length: windows of at most
@@ -340,9 +343,23 @@ int plan_flow(hmf_ctx* c, int zchunk) {
 // worth of per-CTA set-up): small volumes get short chunks, so that their
 // few windows still spread over the SMs.  Chunks are balanced (the deepest
 // volume cut into equal chunks).
+//
+// A pipelined single volume drains its slab pipeline at every replayed
+// graph's end and overlaps slabs within it; there chunks of up to 64 planes
+// measured faster (256^3 tree4: 1.130 ms per iteration at 64 planes, 1.150 at
+// 32), in at least three slabs where those are 20 planes long or more: with
+// two a sweep has little to run beside (us per iteration, before and after:
+// 160 x 160 x 128, four leaves, 173.7 in two slabs, 157.1 in four; 176 x 176 x
+// 80 tree5 199.2 in two, 187.4 in three; 384 x 384 x 60 tree4 630.8 in two,
+// 590.6 in three; but 256 x 256 x 48 tree4 233.3 in one, 238.6 in three).
+// What the overlap hides counts for a tenth of such a plan's cost against a
+// single wave in whole launches (slab_replay; 100 x 128 x 120 tree4, cost ratio
+// 0.93: 144.4 us whole, 126.0 in five slabs; 110^3 four leaves, 1.05: 96.1
+// and 91.7; 84 x 80 x 190 tree5, 1.11: 107.9 and 111.3; 168 x 162 x 62 four
+// leaves, 1.21: 90.9 and 95.9).
 int default_zchunk(const hmf_ctx* c) {
   const int oy = flow_max_out_y(c);
-  const long long slots = std::max(1, c->sm_count) * (c->flow_warps <= 8 ? 2LL : 1LL);  // flow CTAs per SM
+  const long long slots = flow_slots(c);
   long long per_chunk = 0;                                  // CTAs of one z chunk of the largest volume
   int maxz = 1;
   for (const auto& V : c->vols) {
@@ -352,12 +369,11 @@ int default_zchunk(const hmf_ctx* c) {
   }
   // a wave covers about one row of windows only when one volume's chunk
   // takes many waves (a batch of small volumes puts whole volumes in a wave)
-  // A pipelined single volume drains its slab pipeline at every replayed
-  // graph's end and overlaps slabs within it; there chunks of up to 64 planes
-  // measured faster (256^3 tree4: 1.164 ms per iteration at 64 planes against
-  // 1.185 at 43).
   const bool pipelined = c->pipeline && c->vols.size() == 1 && !c->dag;
   const int cap = per_chunk > 8 * slots ? 24 : (pipelined ? 64 : 48);
+  const int third = (maxz + 2) / 3;
+  const bool slabs = pipelined && third >= 20;
+  const int slab_cap = slabs ? third : cap;  // of plans of more than one wave
   int best_z = 1;
   double best = 1e300;
   for (int chunks = 1; chunks <= maxz; ++chunks) {
@@ -369,7 +385,9 @@ int default_zchunk(const hmf_ctx* c) {
       ctas += (long long)((V.vx + hmf::kTmaMaxOutX - 1) / hmf::kTmaMaxOutX) *
               ((V.vy + oy - 1) / oy) * ((V.vz + zv - 1) / zv) * (c->n - 1);
     }
-    const double cost = (double)((ctas + slots - 1) / slots) * (double)(z + 7);
+    if (z > slab_cap && ctas > slots) continue;
+    double cost = (double)((ctas + slots - 1) / slots) * (double)(z + 7);
+    if (slabs && ctas > slots) cost *= 0.9;
     if (cost < best) best = cost, best_z = z;  // ties keep the longer chunk
   }
   return best_z;
@@ -536,21 +554,13 @@ int launch_flow_tma_items(hmf_ctx* c, const hmf::FlowVertexTMA* table, int parit
   if (int rc = maybe_request_stall(c, HMF_STALL_FLOW, s)) return rc;
   const long long units = (long long)n_items * (c->n - 1);
   const dim3 grid((unsigned)((units + c->flow_units - 1) / c->flow_units), 1, 1);
-  const bool multi = c->flow_units > 1;
-  if (c->flow_warps == 16) {
-    if (multi)
-      hmf::flow_tma_kernel<16, true>
-          <<<grid, hmf::FlowTmaShape<16>::kThreads, hmf::FlowTmaShape<16>::kSmemBytes, s>>>(table, fp);
-    else
-      hmf::flow_tma_kernel<16, false>
-          <<<grid, hmf::FlowTmaShape<16>::kThreads, hmf::FlowTmaShape<16>::kSmemBytes, s>>>(table, fp);
-  } else {
-    if (multi)
-      hmf::flow_tma_kernel<8, true><<<grid, hmf::FlowTmaShape<8>::kThreads, hmf::FlowTmaShape<8>::kSmemBytes, s>>>(table, fp);
-    else
-      hmf::flow_tma_kernel<8, false><<<grid, hmf::FlowTmaShape<8>::kThreads, hmf::FlowTmaShape<8>::kSmemBytes, s>>>(table, fp);
-  }
-  CK(cudaGetLastError(), "flow_tma_kernel launch");
+  const bool multi = c->flow_units > 1, tall = c->flow_warps == 16;
+  CK(hmf::launch_waiting(c->overlap_launches,
+                         tall ? (multi ? hmf::flow_tma_kernel<16, true> : hmf::flow_tma_kernel<16, false>)
+                              : (multi ? hmf::flow_tma_kernel<8, true> : hmf::flow_tma_kernel<8, false>),
+                         grid, tall ? hmf::FlowTmaShape<16>::kThreads : hmf::FlowTmaShape<8>::kThreads,
+                         tall ? hmf::FlowTmaShape<16>::kSmemBytes : hmf::FlowTmaShape<8>::kSmemBytes, s, table, fp),
+     "flow_tma_kernel launch");
   ++c->launches;
   return HMF_OK;
 }
@@ -565,25 +575,9 @@ int launch_flow_tma_items(hmf_ctx* c, const hmf::FlowVertexTMA* table, int parit
 constexpr long long kCellVoxels = 350000;
 
 bool cell_path(const hmf_ctx* c) {
-  return c->default_flow && c->pipeline && c->use_tma && c->tree_kind == 0 && !c->dag && c->vols.size() == 1 &&
+  return c->default_flow && !c->tuning && c->pipeline && c->use_tma && c->tree_kind == 0 && !c->dag && c->vols.size() == 1 &&
          c->n <= hmf::kSweepCellMax && !c->gap_on && c->stall_kind < 0 && c->semantics == HMF_SEMANTICS_REF_CUDA &&
          c->total * (c->n - 1) <= kCellVoxels;
-}
-
-// A launch whose prologue may overlap the previous kernel of the stream (the
-// kernel waits for that one's results itself).
-template <class... Params, class... Args>
-cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, int threads, cudaStream_t s, Args... args) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.stream = s;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
 }
 
 int launch_flow_cell(hmf_ctx* c, int parity, cudaStream_t s) {
@@ -591,7 +585,8 @@ int launch_flow_cell(hmf_ctx* c, int parity, cudaStream_t s) {
   hmf::Geometry G{V.vx, V.vy, V.vz, V.pitch, V.plane, V.vol};
   hmf::FlowParams fp{c->step, 1.0f / c->cc, 0, (V.vx + hmf::kCellX - 1) / hmf::kCellX};
   const int tiles = fp.tiles_x * ((V.vy + hmf::kCellY - 1) / hmf::kCellY) * ((V.vz + hmf::kCellZ - 1) / hmf::kCellZ);
-  CK(launch_dependent(hmf::flow_cell_kernel, dim3(tiles, c->n - 1), hmf::kCellThreads, s, c->d_flow[parity], G, fp),
+  CK(hmf::launch_waiting(true, hmf::flow_cell_kernel, dim3(tiles, c->n - 1), hmf::kCellThreads, 0, s, c->d_flow[parity],
+                         G, fp),
      "flow_cell_kernel launch");
   ++c->launches;
   return HMF_OK;
@@ -600,7 +595,7 @@ int launch_flow_cell(hmf_ctx* c, int parity, cudaStream_t s) {
 int launch_sweep_cell(hmf_ctx* c, cudaStream_t s) {
   const dim3 grid((unsigned)((c->geo.vol + hmf::kSweepCellThreads - 1) / hmf::kSweepCellThreads));
   auto launch = [&](auto kernel) {
-    return launch_dependent(kernel, grid, hmf::kSweepCellThreads, s, c->d_tree, c->geo);
+    return hmf::launch_waiting(true, kernel, grid, hmf::kSweepCellThreads, 0, s, c->d_tree, c->geo);
   };
   cudaError_t e = cudaErrorInvalidValue;
   switch (c->n) {
@@ -692,22 +687,22 @@ int launch_tree_bulk_geo(hmf_ctx* c, const hmf::TreeTable* table, const hmf::Geo
   const int grid = (int)std::min<long long>(chunks, (long long)c->sm_count * per_sm);
   if (int rc = maybe_request_stall(c, HMF_STALL_SWEEP, s)) return rc;
   const hmf::GapLog gap = gap_log ? gap_view(c, gap_t) : hmf::GapLog{};
+  auto launch = [&](auto kernel) {
+    return hmf::launch_waiting(c->overlap_launches, kernel, dim3(grid), vc / 4, smem, s, table, G, c->d_error, gap);
+  };
+  cudaError_t e = cudaErrorInvalidValue;
   switch (c->n) {
-#define HMF_TREE_N(N)                                                                        \
-  case N:                                                                                    \
-    if (gap_log)                                                                             \
-      hmf::tree_bulk_n_kernel<N, true><<<grid, vc / 4, smem, s>>>(table, G, c->d_error, gap); \
-    else                                                                                     \
-      hmf::tree_bulk_n_kernel<N, false><<<grid, vc / 4, smem, s>>>(table, G, c->d_error);    \
+#define HMF_TREE_N(N)                                                                                        \
+  case N:                                                                                                    \
+    e = gap_log ? launch(hmf::tree_bulk_n_kernel<N, true>) : launch(hmf::tree_bulk_n_kernel<N, false>);       \
     break;
     HMF_TREE_N(2) HMF_TREE_N(3) HMF_TREE_N(4) HMF_TREE_N(5) HMF_TREE_N(6) HMF_TREE_N(7) HMF_TREE_N(8)
     HMF_TREE_N(9) HMF_TREE_N(10) HMF_TREE_N(11) HMF_TREE_N(12) HMF_TREE_N(13) HMF_TREE_N(14) HMF_TREE_N(15)
     HMF_TREE_N(16)
 #undef HMF_TREE_N
-    default:
-      hmf::tree_bulk_kernel<<<grid, vc / 4, smem, s>>>(table, G, c->d_error, gap);
+    default: e = launch(hmf::tree_bulk_kernel);
   }
-  CK(cudaGetLastError(), "tree_bulk_kernel launch");
+  CK(e, "tree_bulk_kernel launch");
   ++c->launches;
   return HMF_OK;
 }
@@ -831,6 +826,22 @@ bool pipeline_active(const hmf_ctx* c) {
     return false;
   if (c->vols.size() > 1) return true;
   return c->h_fvol[0].zchunk >= 3;
+}
+
+// On the default plan a single volume whose flow CTAs all fit on the GPU at
+// once is iterated in whole launches, each started while the previous one ends
+// (launch_waiting): one wave leaves no idle SMs for a slab's sweep, and every
+// slab costs two launches more.  Time per iteration, pipelined against whole:
+// 128 x 112 x 96 with three leaves 73.2 us against 66.2, 96 x 88 x 72 tree4
+// 72.0 against 66.6, 110 x 100 x 24 tree4 34.7 against 31.8, 128^3 with four
+// leaves (300 CTAs) 119.2 against 118.7, 70^3 with four leaves 36.0 against
+// 37.0; from the second wave on the pipeline wins (160 x 160 x 128, four
+// leaves: 157.1 against 175.6).
+bool slab_replay(const hmf_ctx* c) {
+  if (!pipeline_active(c) || cell_path(c)) return false;
+  if (!c->default_flow || c->vols.size() > 1) return true;
+  const long long units = (long long)c->n_items * (c->n - 1);
+  return (units + c->flow_units - 1) / c->flow_units > flow_slots(c);
 }
 
 // Per-segment sweep tables: the solver's table with every array pointer
@@ -970,18 +981,21 @@ int record_gap_advance(hmf_ctx* c, int n_iter) {
 
 int capture(hmf_ctx* c, int n_iter, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
-  const bool slabs = pipeline_active(c) && !cell_path(c);
+  const bool slabs = slab_replay(c);
   if (slabs)
     if (int rc = prepare_slabs(c, c->stream)) return rc;
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
   long long before = c->launches;
   int rc = HMF_OK;
   if (slabs) rc = record_slab_iterations(c, n_iter);
-  else
+  else {
+    c->overlap_launches = true;
     for (int i = 0; i < n_iter && rc == HMF_OK; ++i) {
       c->gap_t = i;
       rc = record_iteration(c, i & 1, c->stream);
     }
+    c->overlap_launches = false;
+  }
   c->gap_t = 0;
   if (!rc) rc = record_gap_advance(c, n_iter);
   cudaError_t e = cudaStreamEndCapture(c->stream, &g);
@@ -1599,7 +1613,7 @@ int solve_with(hmf_ctx* c, cudaStream_t user, StateLoader load, void* arg) {
     }
     // a DAG's last iteration runs fewer tasks: launched on its own
     const int graphed = c->dag ? std::max(0, c->iterations - 1) : c->iterations;
-    const bool slabs = pipeline_active(c) && !cell_path(c);
+    const bool slabs = slab_replay(c);
     const long long per_iter = slabs ? 2LL * c->n_slabs : 2;
     if (slabs)
       if (int rc2 = upload_slab_tables(c, s)) return rc2;
@@ -1832,8 +1846,8 @@ int hmf_autotune(hmf_ctx* c, void* stream) {
   int rc = HMF_OK;
   DeviceGuard dg(c->device);
   cudaStream_t user = reinterpret_cast<cudaStream_t>(stream);
-  // Each candidate is timed as the solve runs it (graph replay, the slab
-  // pipeline when on): a warm solve captures the plan's graphs, two more are
+  // Each candidate is timed as the solve runs it (graph replay, in whole
+  // launches or through the slab pipeline): a warm solve captures the plan's graphs, two more are
   // timed with events on the caller's stream and the faster counts.  The
   // solves run kTuneIterations iterations, more when the default plan does
   // them in under 2 ms (small volumes), so that launch jitter does not pick
@@ -1846,8 +1860,7 @@ int hmf_autotune(hmf_ctx* c, void* stream) {
   c->iterations = kTuneIterations;
   // what is tuned is the march's plan, for contexts that run it: a small
   // volume that the cell kernels take stays theirs
-  const bool saved_default = c->default_flow;
-  c->default_flow = false;
+  c->tuning = true;
   auto time_plan = [&](int w, int z, int u, float* ms) -> int {
     c->flow_warps = w;
     c->flow_units = u;
@@ -1898,7 +1911,7 @@ int hmf_autotune(hmf_ctx* c, void* stream) {
   }
   c->iterations = saved_iters;
   c->timing = saved_timing;
-  c->default_flow = saved_default;
+  c->tuning = false;
   c->solved = false;
   c->flow_warps = best.warps;
   c->flow_units = best.units;

@@ -23,9 +23,6 @@
 
 namespace hmf {
 
-__device__ __forceinline__ void dependents_may_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_for_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 constexpr int kCellX = 16, kCellY = 8, kCellZ = 4;
 constexpr int kCellThreads = 256;
 

@@ -88,8 +88,10 @@ __global__ void tree_bulk_kernel(const TreeTable* __restrict__ table, const Geom
   uint64_t* bars = reinterpret_cast<uint64_t*>(tb_raw);  // [2], then the stall barrier
   float* stage0 = reinterpret_cast<float*>(tb_raw + 128);
 
+  dependents_may_launch();
   for (int i = threadIdx.x; i < (int)(sizeof(TreeTable) / 4); i += blockDim.x)
     reinterpret_cast<int*>(&T)[i] = reinterpret_cast<const int*>(table)[i];
+  wait_for_previous_grid();
   __syncthreads();  // thread 0 reads the table below
   if (threadIdx.x == 0) {
     const int flag = error_flag ? *(volatile int*)error_flag : 0;
@@ -258,8 +260,10 @@ __global__ void __launch_bounds__(tree_bulk_chunk(N) / 4)
   uint64_t* bars = reinterpret_cast<uint64_t*>(tb_raw);  // [2], then the stall barrier
   float4* stage0 = reinterpret_cast<float4*>(tb_raw + 128);
 
+  dependents_may_launch();
   for (int i = threadIdx.x; i < (int)(sizeof(TreeTable) / 4); i += blockDim.x)
     reinterpret_cast<int*>(&T)[i] = reinterpret_cast<const int*>(table)[i];
+  wait_for_previous_grid();
   if (threadIdx.x == 0) {
     const int flag = error_flag ? *(volatile int*)error_flag : 0;
     abort_cta = flag & 2;

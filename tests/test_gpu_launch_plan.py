@@ -1,0 +1,61 @@
+"""How a single volume's iterations are launched on the default plan: whole
+launches that overlap their successors while the flow step is resident at
+once, the slab pipeline (in at least three slabs) from there on.  Both give
+the oracle's results bit for bit, over odd and long iteration counts and with
+the convergence log.  GPU only."""
+import numpy as np
+import pytest
+
+from robartsvtk_gb300 import HMFSolver
+from robartsvtk_gb300.synthetic import random_tree_problem
+from tests.test_gpu_parity import assert_same, oracle, run_gpu
+
+pytestmark = pytest.mark.gpu
+
+FLAT3 = [-1, 0, 0, 0]
+TREE8 = [-1, 0, 0, 1, 1, 2, 2, 3, 3, 4, 4, 5, 5, 6, 6]
+
+
+@pytest.mark.parametrize("dims,parent,iterations,slabs", [
+    ((64, 60, 48), FLAT3, 33, 1),         # one wave: 144 units
+    ((61, 59, 47), FLAT3, 70, 1),         # odd axes, two long replays
+    ((300, 9, 50), [-1, 0, 1, 1], 5, 1),  # windows in x only
+    ((100, 80, 60), TREE8, 5, 3),         # 60 planes in thirds
+    ((100, 80, 59), TREE8, 4, 3),         # the last slab shorter
+    ((130, 120, 30), TREE8, 3, 2),        # too thin for thirds of 20 planes: two slabs of 15
+    ((112, 112, 60), [-1, 0, 1, 1, 1, 0, 0], 2, 5),  # five slabs cost less than one wave
+    ((168, 162, 62), [-1, 0, 0, 0, 0], 2, 1),        # one wave costs less than slabs
+])
+def test_default_plan(dims, parent, iterations, slabs):
+    w = random_tree_problem(11, dims, parent, iterations=iterations, smooth_nodes=(1,))
+    r = run_gpu(w)
+    assert_same(r, oracle(w), str(dims))
+    assert r["stats"]["launches"] == 1 + 2 * slabs * iterations
+
+
+def test_whole_launches_with_the_log_and_continued():
+    """The log's entries and the state after rounds of a continued solve are
+    those of launches one by one (timing mode records no graphs)."""
+    w = random_tree_problem(12, (60, 58, 52), FLAT3, iterations=0, smooth_nodes=(2,))
+    out = []
+    for timing in (False, True):
+        with HMFSolver(w.dims, w.parent) as s:
+            s.set_timing(timing)
+            s.set_convergence_log(True)
+            for leaf, d in w.data.items():
+                s.set_data(leaf, d)
+            for v, S in w.smooth.items():
+                s.set_smoothness(v, S)
+            for v, a in w.alpha.items():
+                s.set_smoothness_scalar(v, a)
+            logs = []
+            for i, k in enumerate((35, 1, 4)):
+                s.set_params(k, w.step, w.cc)
+                s.solve() if i == 0 else s.solve_continue()
+                logs.append(s.convergence())
+            out.append((logs, [s.labels(v) for v in range(1, len(w.parent))], [s.sink(v) for v in range(len(w.parent))]))
+    for a, b in zip(out[0][0], out[1][0]):
+        assert len(a["max"]) and np.array_equal(a["max"], b["max"])
+        np.testing.assert_allclose(a["mean"], b["mean"], rtol=1e-6)
+    for a, b in zip(out[0][1] + out[0][2], out[1][1] + out[1][2]):
+        assert np.array_equal(a, b)
