@@ -731,7 +731,7 @@ int launch_dag_sweep(hmf_ctx* c, cudaStream_t s) {
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, hmf::kDagNVc, smem) != cudaSuccess || per < 1)
         per = 1;
       const int grid = (int)std::max<long long>(1, std::min<long long>(chunks, (long long)c->sm_count * per));
-      kernel<<<grid, hmf::kDagNVc, smem, s>>>(c->h_dagreg, c->geo.vol, c->dag_last ? 1 : 0, c->d_error);
+      kernel<<<grid, hmf::kDagNVc, smem, s>>>(c->h_dagreg, c->d_dag, c->geo.vol, c->dag_last ? 1 : 0, c->d_error);
     };
     switch (c->n) {
       case 2: launch(hmf::dag_bulk_n_kernel<2>); break;
@@ -1095,7 +1095,6 @@ int prepare_dag_table(hmf_ctx* c, cudaStream_t s, const Staged& in) {
     R.inc[i] = E.inc;
     R.label[i] = E.label;
     R.div[i] = E.div;
-    R.data[i] = E.data;
     R.k[i] = E.k;
     if (E.leaf) R.leaf_mask |= 1u << i;
     R.n_in[i] = E.n_in;

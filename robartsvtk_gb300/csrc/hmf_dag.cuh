@@ -344,7 +344,8 @@ __host__ __device__ constexpr int dag_bulk_n_smem_bytes(int N) {
 
 template <int N>
 __global__ void __launch_bounds__(kDagNVc)
-    dag_bulk_n_kernel(const __grid_constant__ DagRegParams P, long long n_vox, int last, int* __restrict__ error_flag) {
+    dag_bulk_n_kernel(const __grid_constant__ DagRegParams P, const DagTable* __restrict__ table, long long n_vox,
+                      int last, int* __restrict__ error_flag) {
   constexpr int A = dag_bulk_n_arrays(N);
   constexpr int VC = kDagNVc;
   constexpr int ROOT = 5 * (N - 1);
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(kDagNVc)
     asrc = kind == 0 ? P.sink[e] : kind == 1 ? P.inc[e] : kind == 2 ? P.div[e] : P.label[e];
   } else if (ta < ROOT) {
     const int e = ta - 4 * (N - 1) + 1;
-    if ((P.leaf_mask >> e) & 1u) asrc = P.data[e];
+    if ((P.leaf_mask >> e) & 1u) asrc = table->e[e].data;
   } else if (ta == ROOT) {
     asrc = P.sink[0];
   }

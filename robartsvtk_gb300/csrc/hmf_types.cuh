@@ -88,13 +88,14 @@ struct DagTable {
 // The graph of dag_bulk_n_kernel<N> (N <= 8 entries, no repeated edge), in
 // kernel parameters: entry e's staged arrays, its parents as a bit mask with
 // per-pair weights, and its parents in in-edge order for the push-down sum.
+// Only what stays for the life of a captured launch: the data terms, which may
+// lie elsewhere at the next solve, are found through the graph table.
 constexpr int kDagRegMax = 8;
 struct DagRegParams {
   float* sink[kDagRegMax];  // entry 0: the root's source
   float* inc[kDagRegMax];
   float* label[kDagRegMax];
   const float* div[kDagRegMax];
-  const float* data[kDagRegMax];
   float k[kDagRegMax];                    // branch reset weights
   float wup[kDagRegMax][kDagRegMax];      // [child][parent] push-up weight
   float wdown_ord[kDagRegMax][kDagRegMax];  // [child][j] push-down weight of its j-th in-edge
