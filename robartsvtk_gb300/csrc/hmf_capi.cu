@@ -369,7 +369,7 @@ int default_zchunk(const hmf_ctx* c) {
   }
   // a wave covers about one row of windows only when one volume's chunk
   // takes many waves (a batch of small volumes puts whole volumes in a wave)
-  const bool pipelined = c->pipeline && c->vols.size() == 1 && !c->dag;
+  const bool pipelined = c->pipeline && c->vols.size() == 1 && (!c->dag || c->n <= hmf::kDagRegMax);
   const int cap = per_chunk > 8 * slots ? 24 : (pipelined ? 64 : 48);
   const int third = (maxz + 2) / 3;
   const bool slabs = pipelined && third >= 20;
@@ -720,32 +720,47 @@ int dag_grid(hmf_ctx* c, const void* kernel, size_t smem) {
   return (int)std::max<long long>(1, std::min<long long>(blocks, (long long)c->sm_count * per));
 }
 
+// Whether the graph's sweep is dag_bulk_n_kernel.
+bool dag_in_parameters(const hmf_ctx* c) { return !c->dag_simple && !c->dag_generic && c->dag_reg_ok; }
+
+// dag_bulk_n_kernel over the elements [base, base + vol).
+int launch_dag_elements(hmf_ctx* c, long long base, long long vol, cudaStream_t s) {
+  const int smem = hmf::dag_bulk_n_smem_bytes(c->n);
+  const long long chunks = (vol + hmf::kDagNVc - 1) / hmf::kDagNVc;
+  hmf::DagRegParams P = c->h_dagreg;
+  for (int e = 0; e < c->n; ++e) {
+    if (P.sink[e]) P.sink[e] += base;
+    if (P.inc[e]) P.inc[e] += base;
+    if (P.label[e]) P.label[e] += base;
+    if (P.div[e]) P.div[e] += base;
+  }
+  auto launch = [&](auto kernel) {
+    int per = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, hmf::kDagNVc, smem) != cudaSuccess || per < 1)
+      per = 1;
+    const int grid = (int)std::max<long long>(1, std::min<long long>(chunks, (long long)c->sm_count * per));
+    return hmf::launch_waiting(c->overlap_launches, kernel, dim3(grid), hmf::kDagNVc, smem, s, P, c->d_dag, base, vol,
+                               c->dag_last ? 1 : 0, c->d_error);
+  };
+  cudaError_t e = cudaErrorInvalidValue;
+  switch (c->n) {
+    case 2: e = launch(hmf::dag_bulk_n_kernel<2>); break;
+    case 3: e = launch(hmf::dag_bulk_n_kernel<3>); break;
+    case 4: e = launch(hmf::dag_bulk_n_kernel<4>); break;
+    case 5: e = launch(hmf::dag_bulk_n_kernel<5>); break;
+    case 6: e = launch(hmf::dag_bulk_n_kernel<6>); break;
+    case 7: e = launch(hmf::dag_bulk_n_kernel<7>); break;
+    default: e = launch(hmf::dag_bulk_n_kernel<8>); break;
+  }
+  CK(e, "dag_bulk_n_kernel launch");
+  ++c->launches;
+  return HMF_OK;
+}
+
 int launch_dag_sweep(hmf_ctx* c, cudaStream_t s) {
   if (!c->dag_simple)
     if (int rc = maybe_request_stall(c, HMF_STALL_SWEEP, s)) return rc;
-  if (!c->dag_simple && !c->dag_generic && c->dag_reg_ok) {
-    const int smem = hmf::dag_bulk_n_smem_bytes(c->n);
-    const long long chunks = (c->geo.vol + hmf::kDagNVc - 1) / hmf::kDagNVc;
-    auto launch = [&](auto kernel) {
-      int per = 1;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, hmf::kDagNVc, smem) != cudaSuccess || per < 1)
-        per = 1;
-      const int grid = (int)std::max<long long>(1, std::min<long long>(chunks, (long long)c->sm_count * per));
-      kernel<<<grid, hmf::kDagNVc, smem, s>>>(c->h_dagreg, c->d_dag, c->geo.vol, c->dag_last ? 1 : 0, c->d_error);
-    };
-    switch (c->n) {
-      case 2: launch(hmf::dag_bulk_n_kernel<2>); break;
-      case 3: launch(hmf::dag_bulk_n_kernel<3>); break;
-      case 4: launch(hmf::dag_bulk_n_kernel<4>); break;
-      case 5: launch(hmf::dag_bulk_n_kernel<5>); break;
-      case 6: launch(hmf::dag_bulk_n_kernel<6>); break;
-      case 7: launch(hmf::dag_bulk_n_kernel<7>); break;
-      default: launch(hmf::dag_bulk_n_kernel<8>); break;
-    }
-    CK(cudaGetLastError(), "dag_bulk_n_kernel launch");
-    ++c->launches;
-    return HMF_OK;
-  }
+  if (dag_in_parameters(c)) return launch_dag_elements(c, 0, c->geo.vol, s);
   if (!c->dag_simple) {
     const int A = hmf::dag_bulk_arrays(c->n, (int)c->leaves.size());
     const int vc = hmf::dag_bulk_chunk(A);
@@ -796,7 +811,8 @@ int record_iteration(hmf_ctx* c, int parity, cudaStream_t s) {
 }
 
 // ---- z-slab pipeline of the replayed iterations ---------------------------
-// With the pipeline on (hmf_set_pipeline) a single volume's iteration is cut
+// With the pipeline on (hmf_set_pipeline) a single volume's iteration (of a
+// label tree, or of a graph whose sweep is dag_bulk_n_kernel) is cut
 // at the flow plan's z chunks into slabs: the flow launch of a slab runs its
 // chunk's work items, the sweep launch of a slab its planes' elements, each
 // a graph node with only the dependencies the stencil needs --
@@ -820,13 +836,16 @@ int record_iteration(hmf_ctx* c, int parity, cudaStream_t s) {
 // previous launch, and the groups' flows and sweeps overlap freely.
 constexpr int kBatchGroups = 6;
 
-bool pipeline_active(const hmf_ctx* c) {
-  if (!c->pipeline || c->dag || !c->use_tma || c->tree_kind != 0 || c->semantics != HMF_SEMANTICS_REF_CUDA ||
-      c->n_items <= 0 || c->h_fvol.empty())
+bool slabs_possible(const hmf_ctx* c) {
+  if (!c->pipeline || !c->use_tma || c->semantics != HMF_SEMANTICS_REF_CUDA || c->n_items <= 0 || c->h_fvol.empty())
     return false;
+  if (c->dag ? !dag_in_parameters(c) : c->tree_kind != 0) return false;
   if (c->vols.size() > 1) return true;
   return c->h_fvol[0].zchunk >= 3;
 }
+
+// The pipeline as hmf_get_pipeline reports it: a label tree's.
+bool pipeline_active(const hmf_ctx* c) { return !c->dag && slabs_possible(c); }
 
 // On the default plan a single volume whose flow CTAs all fit on the GPU at
 // once is iterated in whole launches, each started while the previous one ends
@@ -838,7 +857,7 @@ bool pipeline_active(const hmf_ctx* c) {
 // 37.0; from the second wave on the pipeline wins (160 x 160 x 128, four
 // leaves: 157.1 against 175.6).
 bool slab_replay(const hmf_ctx* c) {
-  if (!pipeline_active(c) || cell_path(c)) return false;
+  if (!slabs_possible(c) || cell_path(c)) return false;
   if (!c->default_flow || c->vols.size() > 1) return true;
   const long long units = (long long)c->n_items * (c->n - 1);
   return (units + c->flow_units - 1) / c->flow_units > flow_slots(c);
@@ -849,6 +868,7 @@ bool slab_replay(const hmf_ctx* c) {
 // so they are written before every pipelined solve, into the array the
 // graphs point at).
 int upload_slab_tables(hmf_ctx* c, cudaStream_t s) {
+  if (c->dag) return HMF_OK;  // (its slabs' launches carry their pointers)
   const int K = c->n_slabs;
   c->h_tree_slabs.assign(K, c->h_tree);
   for (int k = 0; k < K; ++k) {
@@ -962,7 +982,9 @@ int record_slab_iterations(hmf_ctx* c, int n_iter) {
       cudaStream_t st = c->slab_streams[k];
       for (int j = std::max(0, k - c->seg_neighbours); j <= std::min(K - 1, k + c->seg_neighbours); ++j)
         if (j != k) CK(cudaStreamWaitEvent(st, c->slab_ev_flow[j], 0), "cudaStreamWaitEvent(flow)");
-      if (int rc = launch_tree_bulk_geo(c, c->d_tree_slabs + k, c->slab_geo[k], st, c->gap_on, t)) return rc;
+      if (int rc = c->dag ? launch_dag_elements(c, c->seg_base[k], c->slab_geo[k].vol, st)
+                          : launch_tree_bulk_geo(c, c->d_tree_slabs + k, c->slab_geo[k], st, c->gap_on, t))
+        return rc;
       CK(cudaEventRecord(c->slab_ev_sweep[k], st), "cudaEventRecord(sweep)");
     }
   }
@@ -1607,7 +1629,7 @@ int solve_with(hmf_ctx* c, cudaStream_t user, StateLoader load, void* arg) {
       if (!rc) rc = capture(c, 1, &c->graph_one);
       // a pipelined solve replays several iterations per graph, so that the
       // pipeline drains (at a graph's end) rarely
-      if (!rc && (pipeline_active(c) || cell_path(c))) rc = capture(c, kPipelineIterations, &c->graph_many);
+      if (!rc && (slabs_possible(c) || cell_path(c))) rc = capture(c, kPipelineIterations, &c->graph_many);
       if (rc) return rc;
     }
     // a DAG's last iteration runs fewer tasks: launched on its own

@@ -335,7 +335,8 @@ __global__ void dag_bulk_kernel(const DagTable* __restrict__ table, long long n_
 // graph in kernel parameters, staged slots at compile-time offsets (entry
 // e >= 1: sink 4(e-1), source +1, divergence +2, label +3, data term
 // 4(N-1) + e-1; the root's source 5(N-1)), so the per-voxel program reads no
-// table.  Same arithmetic and order as dag_bulk_kernel.
+// table.  Same arithmetic and order as dag_bulk_kernel.  P's arrays begin at
+// the launch's first element, element `base` of the whole volume.
 constexpr int kDagNVc = 256;
 __host__ __device__ constexpr int dag_bulk_n_arrays(int N) { return 5 * (N - 1) + 1; }
 __host__ __device__ constexpr int dag_bulk_n_smem_bytes(int N) {
@@ -344,8 +345,8 @@ __host__ __device__ constexpr int dag_bulk_n_smem_bytes(int N) {
 
 template <int N>
 __global__ void __launch_bounds__(kDagNVc)
-    dag_bulk_n_kernel(const __grid_constant__ DagRegParams P, const DagTable* __restrict__ table, long long n_vox,
-                      int last, int* __restrict__ error_flag) {
+    dag_bulk_n_kernel(const __grid_constant__ DagRegParams P, const DagTable* __restrict__ table, long long base,
+                      long long n_vox, int last, int* __restrict__ error_flag) {
   constexpr int A = dag_bulk_n_arrays(N);
   constexpr int VC = kDagNVc;
   constexpr int ROOT = 5 * (N - 1);
@@ -353,6 +354,8 @@ __global__ void __launch_bounds__(kDagNVc)
   extern __shared__ __align__(128) unsigned char dn_raw[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(dn_raw);
   float* const stage0 = reinterpret_cast<float*>(dn_raw + 128);
+  dependents_may_launch();
+  wait_for_previous_grid();
   if (threadIdx.x == 0) {
     const int flag = error_flag ? *(volatile int*)error_flag : 0;
     abort_cta = flag & 2;
@@ -387,7 +390,7 @@ __global__ void __launch_bounds__(kDagNVc)
     asrc = kind == 0 ? P.sink[e] : kind == 1 ? P.inc[e] : kind == 2 ? P.div[e] : P.label[e];
   } else if (ta < ROOT) {
     const int e = ta - 4 * (N - 1) + 1;
-    if ((P.leaf_mask >> e) & 1u) asrc = table->e[e].data;
+    if ((P.leaf_mask >> e) & 1u) asrc = table->e[e].data + base;
   } else if (ta == ROOT) {
     asrc = P.sink[0];
   }

@@ -6,8 +6,9 @@ the convergence log.  GPU only."""
 import numpy as np
 import pytest
 
-from robartsvtk_gb300 import HMFSolver
+from robartsvtk_gb300 import DAGSolver, HMFSolver
 from robartsvtk_gb300.synthetic import random_tree_problem
+from tests.test_gpu_dag import assert_exact, oracle_solve, random_dag
 from tests.test_gpu_parity import assert_same, oracle, run_gpu
 
 pytestmark = pytest.mark.gpu
@@ -59,3 +60,35 @@ def test_whole_launches_with_the_log_and_continued():
         np.testing.assert_allclose(a["mean"], b["mean"], rtol=1e-6)
     for a, b in zip(out[0][1] + out[0][2], out[1][1] + out[1][2]):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("dims,zchunk,iterations,slabs", [
+    ((112, 112, 60), 0, 3, 5),   # the default plan's slabs
+    ((30, 20, 24), 6, 35, 4),    # a long replay
+    ((29, 21, 23), 5, 4, 5),     # odd axes, the last slab shorter
+    ((29, 21, 23), 2, 4, 1),     # chunks too thin for slabs
+    ((40, 30, 20), 0, 5, 1),     # one wave
+])
+def test_graph_in_slabs(dims, zchunk, iterations, slabs):
+    """A graph's iterations; its last one runs fewer tasks, in whole launches.
+    The second solve's inputs lie elsewhere."""
+    import torch
+    edges = [(0, 1), (1, 2), (1, 3), (0, 4), (4, 5), (4, 6), (4, 3)]
+    w = random_dag(19, dims, 7, edges, iterations=iterations, smooth_nodes=(1, 4))
+    o = oracle_solve(w)
+    keep = []
+    with DAGSolver(w.dims, w.n, w.edges, w.weights) as s:
+        s.set_zchunk(zchunk)
+        for v, S in w.smooth.items():
+            s.set_smoothness(v, S)
+        for v, a in w.alpha.items():
+            s.set_smoothness_scalar(v, a)
+        s.set_params(w.iterations, w.step, w.cc)
+        for _ in range(2):
+            for leaf, d in w.data.items():
+                keep.append(torch.from_numpy(np.ascontiguousarray(d)).cuda())
+                s.set_data(leaf, keep[-1])
+            s.solve()
+            assert_exact({"u": {v: s.labels(v) for v in range(1, w.n)}, "sink": {v: s.sink(v) for v in range(w.n)}}, o,
+                         str(dims))
+            assert s.stats()["launches"] == 1 + 2 * slabs * (iterations - 1) + 2
