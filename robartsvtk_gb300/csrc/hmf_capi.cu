@@ -54,7 +54,10 @@ thread_local std::string g_create_error;
 constexpr int kMaxDim = 1 << 30;
 
 constexpr int kTX = 32, kTY = 8;
-constexpr int kPipelineIterations = 32;  // iterations per replayed graph of a pipelined solve (even)
+// Iterations per replayed graph, longest first; each is recorded when a solve
+// first takes it.  Overlapping slabs and launches drain at a graph's end, and
+// a graph's recording grows with its length.
+constexpr int kReplay[hmf_ctx::kReplays] = {32, 8, 2, 1};
 constexpr int kTuneIterations = 8;      // iterations of each solve the autotuner times
 constexpr int kMaxFlowUnits = 64;       // units (window-vertex marches) one flow CTA may take
 constexpr int kTreeThreads = 256;
@@ -892,7 +895,7 @@ int upload_slab_tables(hmf_ctx* c, cudaStream_t s) {
 // Segments of the current plan (one per z chunk of a single volume, or
 // groups of a batch's volumes), their tables' device array, streams and
 // events (made when the graphs are captured).
-int prepare_slabs(hmf_ctx* c, cudaStream_t s) {
+int prepare_slabs(hmf_ctx* c) {
   c->seg_first_item.clear();
   c->seg_items.clear();
   c->seg_base.clear();
@@ -948,7 +951,6 @@ int prepare_slabs(hmf_ctx* c, cudaStream_t s) {
     CK(cudaMalloc(&c->d_tree_slabs, sizeof(hmf::TreeTable) * K), "cudaMalloc(slab tables)");
   }
   c->n_slabs = K;
-  if (int rc = upload_slab_tables(c, s)) return rc;
   while ((int)c->slab_streams.size() < K) {
     cudaStream_t st = nullptr;
     CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate(slab)");
@@ -1005,7 +1007,7 @@ int capture(hmf_ctx* c, int n_iter, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
   const bool slabs = slab_replay(c);
   if (slabs)
-    if (int rc = prepare_slabs(c, c->stream)) return rc;
+    if (int rc = prepare_slabs(c)) return rc;
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
   long long before = c->launches;
   int rc = HMF_OK;
@@ -1035,10 +1037,10 @@ int capture(hmf_ctx* c, int n_iter, cudaGraphExec_t* out) {
 
 void drop_graphs(hmf_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
-  if (c->graph_pair) cudaGraphExecDestroy(c->graph_pair);
-  if (c->graph_one) cudaGraphExecDestroy(c->graph_one);
-  if (c->graph_many) cudaGraphExecDestroy(c->graph_many);
-  c->graph_pair = c->graph_one = c->graph_many = nullptr;
+  for (auto& g : c->replay) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
 }
 
 int timed(hmf_ctx* c, int kind, cudaStream_t s, int (*fn)(hmf_ctx*, cudaStream_t, int), int arg) {
@@ -1624,33 +1626,23 @@ int solve_with(hmf_ctx* c, cudaStream_t user, StateLoader load, void* arg) {
       if (rc) return rc;
     }
   } else {
-    if (!c->graph_pair) {
-      rc = capture(c, 2, &c->graph_pair);
-      if (!rc) rc = capture(c, 1, &c->graph_one);
-      // a pipelined solve replays several iterations per graph, so that the
-      // pipeline drains (at a graph's end) rarely
-      if (!rc && (slabs_possible(c) || cell_path(c))) rc = capture(c, kPipelineIterations, &c->graph_many);
-      if (rc) return rc;
-    }
     // a DAG's last iteration runs fewer tasks: launched on its own
     const int graphed = c->dag ? std::max(0, c->iterations - 1) : c->iterations;
     const bool slabs = slab_replay(c);
-    const long long per_iter = slabs ? 2LL * c->n_slabs : 2;
-    if (slabs)
-      if (int rc2 = upload_slab_tables(c, s)) return rc2;
-    int it0 = 0;
-    if (c->graph_many)
-      for (; it0 + kPipelineIterations <= graphed; it0 += kPipelineIterations) {
-        CK(cudaGraphLaunch(c->graph_many, s), "cudaGraphLaunch");
-        c->launches += per_iter * kPipelineIterations;
+    bool tables_written = false;
+    int left = graphed;
+    for (int k = 0; k < hmf_ctx::kReplays; left %= kReplay[k++]) {
+      if (left < kReplay[k]) continue;
+      // (recorded here, a shorter graph's recording runs beside the longer ones)
+      if (!c->replay[k])
+        if (rc = capture(c, kReplay[k], &c->replay[k])) return rc;
+      if (slabs && !tables_written)
+        if (rc = upload_slab_tables(c, s)) return rc;
+      tables_written = true;
+      for (int n = left / kReplay[k]; n > 0; --n) {
+        CK(cudaGraphLaunch(c->replay[k], s), "cudaGraphLaunch");
+        c->launches += (slabs ? 2LL * c->n_slabs : 2) * kReplay[k];
       }
-    for (int it = it0; it + 1 < graphed; it += 2) {
-      CK(cudaGraphLaunch(c->graph_pair, s), "cudaGraphLaunch");
-      c->launches += 2 * per_iter;
-    }
-    if ((graphed - it0) & 1) {
-      CK(cudaGraphLaunch(c->graph_one, s), "cudaGraphLaunch");
-      c->launches += per_iter;
     }
     if (c->dag && c->iterations > 0) {
       rc = launch_flow(c, graphed & 1, s);
@@ -1723,9 +1715,8 @@ int hmf_destroy(hmf_ctx* c) {
   DeviceGuard dg(c->device);
   paged_free(c);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  if (c->graph_pair) cudaGraphExecDestroy(c->graph_pair);
-  if (c->graph_one) cudaGraphExecDestroy(c->graph_one);
-  if (c->graph_many) cudaGraphExecDestroy(c->graph_many);
+  for (auto g : c->replay)
+    if (g) cudaGraphExecDestroy(g);
   if (c->d_tree_slabs) cudaFree(c->d_tree_slabs);
   for (auto st : c->slab_streams) cudaStreamDestroy(st);
   for (auto ev : c->slab_ev_flow) cudaEventDestroy(ev);

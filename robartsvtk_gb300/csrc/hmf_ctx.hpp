@@ -88,9 +88,8 @@ struct hmf_ctx {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_join = nullptr;
   cudaEvent_t ev_t0 = nullptr, ev_t1 = nullptr;
-  cudaGraphExec_t graph_pair = nullptr;  // two iterations (both flow parities)
-  cudaGraphExec_t graph_one = nullptr;   // one iteration, parity 0
-  cudaGraphExec_t graph_many = nullptr;  // pipelined solves: several iterations per replay
+  static constexpr int kReplays = 4;
+  cudaGraphExec_t replay[kReplays] = {};  // recorded iterations, by length (the shortest, one, last)
 
   // z-slab pipeline of the replayed iterations (hmf_set_pipeline)
   bool pipeline = true;
