@@ -6,17 +6,28 @@
 // A persistent CTA walks chunks of 256 consecutive voxels of the pitched
 // layout (padding columns included: their values are finite and never read
 // back).  For every chunk lane v of warp 0 issues vertex v's cp.async.bulk
-// copies, one per input array -- per vertex the sweep parts of the later state's sink and label
-// adjoints, the later flow reverse's gb, the sink and label before the
-// iteration, the sink and divergence after it, the data term and the
-// accumulated data-term gradient (double) -- into one of two shared-memory
-// stages; a stage is refilled as soon as its chunk has been read into
-// registers, so two chunks stream in while one is reversed.  Stage
-// slots sit at fixed [quantity][vertex] positions (absent quantities are not
-// copied and not read), so every shared-memory offset is a compile-time
-// constant; one thread reverses one voxel with all per-vertex values in
-// registers.  When the vertex ids are in pre-order (PRE), the sink pass runs
-// in compile-time vertex order; otherwise runtime vertices (parents,
+// copies, one per input array -- per vertex the sweep parts of the later
+// state's sink and label adjoints, the later flow reverse's gb, the sink and
+// label before the iteration, the sink and divergence after it, and the data
+// term -- into one of two shared-memory stages; a stage is refilled as soon as
+// its chunk has been read into registers, so two chunks stream in while one is
+// reversed.  Stage slots sit at fixed positions, so that every shared-memory
+// offset is a compile-time constant (but the last vertex's, where the root's
+// unused slots are its own and the root's id is not known); one thread
+// reverses one voxel with all per-vertex values in registers.
+//
+// The kernel is bound by the latency of a chunk (copies, then a serial pass
+// over the vertices), so what counts is CTAs per SM, and those are limited by
+// the stages: only arrays that exist have a slot (7 N - 4 per stage), and the
+// accumulated data-term gradient (double) is not staged but added to in place
+// by the voxels whose sink lies at its data term -- one addition per element
+// and launch, so in no other order than before.  Per launch: 96 x 88 x 72, 7
+// vertices 73.9 us with 1 CTA per SM (ten slots per vertex), 38.7 us with 2;
+// 128^3, 5 vertices 74.0 us with 2, 62.1 us with 3 (5.9 TB/s of copies and
+// stores, part of them in L2).
+//
+// When the vertex ids are in pre-order (PRE), the root is 0 and the sink pass
+// runs in compile-time vertex order; otherwise runtime vertices (parents,
 // children, pre-order positions) are reached through predicated selects.
 // FLAT trees (root 0, every other vertex a leaf under it) also have their
 // parents at compile time, so no select or parent test is left; the
@@ -30,11 +41,18 @@ namespace hmf {
 
 constexpr int kSwVc = 256;     // voxels per chunk = threads per CTA
 constexpr int kSwMaxN = 8;
-constexpr int kSwKinds = 10;   // float slots per vertex: 8 quantities + one double (2 floats)
 
-enum { kSwSBN = 0, kSwUB, kSwGB, kSwAS, kSwAU, kSwBS, kSwBD, kSwD, kSwDB };  // kSwDB: double, 2 slots
+// Staged quantities: the first three of every vertex (the later sink of a
+// branch or the root, the data term of a leaf), the others of every vertex but
+// the root -- whose slot there the last vertex takes.
+enum { kSwSBN = 0, kSwBS, kSwASD, kSwUB, kSwGB, kSwAU, kSwBD };
+__host__ __device__ constexpr int adj_sweep_slots(int N) { return 3 * N + 4 * (N - 1); }
+template <int N>
+__device__ __forceinline__ int sw_slot(int kind, int v, int root) {
+  return kind < 3 ? kind * N + v : 3 * N + (kind - 3) * (N - 1) + (v == N - 1 ? root : v);
+}
 
-__host__ __device__ constexpr int adj_sweep_smem_bytes(int N) { return 128 + 2 * kSwKinds * N * kSwVc * 4; }
+__host__ __device__ constexpr int adj_sweep_smem_bytes(int N) { return 128 + 2 * adj_sweep_slots(N) * kSwVc * 4; }
 
 template <int N>
 __device__ __forceinline__ float sw_sel(const float (&a)[N], int v) {
@@ -53,14 +71,14 @@ __device__ __forceinline__ void sw_add(float (&a)[N], int v, float x) {
 }
 
 template <int N, bool PRE, bool FLAT>
-__global__ void __launch_bounds__(kSwVc) adj_sweep_kernel(const AdjTree* __restrict__ table, const Geometry G,
+__global__ void __launch_bounds__(kSwVc, N <= 5 ? 3 : 2) adj_sweep_kernel(const AdjTree* __restrict__ table, const Geometry G,
                                                           const AdjSweep S, int* __restrict__ error_flag) {
   __shared__ AdjTree T;
   __shared__ int abort_cta, stall_cta, stop_cta;
   extern __shared__ __align__(128) unsigned char sw_raw[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(sw_raw);  // [2], then the stall barrier
   float* stage0 = reinterpret_cast<float*>(sw_raw + 128);
-  constexpr int kStage = kSwKinds * N * kSwVc;  // floats per stage
+  constexpr int kStage = adj_sweep_slots(N) * kSwVc;  // floats per stage
 
   dependents_may_launch();
   for (int i = threadIdx.x; i < (int)(sizeof(AdjTree) / 4); i += blockDim.x)
@@ -84,7 +102,7 @@ __global__ void __launch_bounds__(kSwVc) adj_sweep_kernel(const AdjTree* __restr
   if (abort_cta) return;
 
   static_assert(!FLAT || PRE, "a flat tree with root 0 has its ids in pre-order");
-  const int root = FLAT ? 0 : T.root;
+  const int root = PRE ? 0 : T.root;
   auto par = [&](int v) { return FLAT ? (v == 0 ? -1 : 0) : T.parent[v]; };
   auto is_leaf = [&](int v) { return FLAT ? v != 0 : T.n_kids[v] == 0; };
   const float cc = T.cc, icc = T.icc, step = T.step, step_icc = T.step * T.icc;
@@ -99,26 +117,24 @@ __global__ void __launch_bounds__(kSwVc) adj_sweep_kernel(const AdjTree* __restr
     uint64_t* bar = &bars[s];
     float* dst = stage0 + (size_t)s * kStage;
     {
-      const bool nr = v != root, leaf = is_leaf(v);
-      mbar_expect_tx(bar, len * 4 * (3 + (nr ? 4 : 0)) + (leaf ? len * 8 : 0));
+      const bool nr = v != root;
+      mbar_expect_tx(bar, len * 4 * (3 + (nr ? 4 : 0)));
     }
     auto ld = [&](int kind, int v, const float* src) {
-      bulk_load(dst + (size_t)(kind * N + v) * kSwVc, src + v0, len * 4, bar);
+      bulk_load(dst + sw_slot<N>(kind, v, root) * kSwVc, src + v0, len * 4, bar);
     };
     {
       const long long b = T.sbase[v];
       const bool nr = v != root, leaf = is_leaf(v);
       ld(kSwSBN, v, S.sbn + v * arr);
       ld(kSwBS, v, S.stB + b * arr);
-      if (leaf) ld(kSwD, v, T.data[v]);
-      else ld(kSwAS, v, S.stA + b * arr);
+      ld(kSwASD, v, leaf ? T.data[v] : S.stA + b * arr);
       if (nr) {
         ld(kSwUB, v, S.ubn + v * arr);
         ld(kSwGB, v, S.gbn + v * arr);
         ld(kSwAU, v, S.stA + (b + kAdjLabel) * arr);
         ld(kSwBD, v, S.stB + (b + kAdjDiv) * arr);
       }
-      if (leaf) bulk_load(dst + (size_t)(kSwDB * N + 2 * v) * kSwVc, T.Db[v] + v0, len * 8, bar);
     }
   };
 
@@ -145,23 +161,20 @@ __global__ void __launch_bounds__(kSwVc) adj_sweep_kernel(const AdjTree* __restr
     const int len = (int)min((long long)kSwVc, G.vol - v0);
     const int q = threadIdx.x;
     float SBN[N], UB[N], GB[N], AS[N], AU[N], BS[N], BD[N], D[N];
-    double DB[N];
-    bool hit[N];
     if (q < len) {
-      auto at = [&](int kind, int v) { return st[(kind * N + v) * kSwVc + q]; };
+      auto at = [&](int kind, int v) { return st[sw_slot<N>(kind, v, root) * kSwVc + q]; };
 #pragma unroll
       for (int v = 0; v < N; ++v) {
         const bool nr = v != root, leaf = is_leaf(v);
         SBN[v] = at(kSwSBN, v);
         BS[v] = at(kSwBS, v);
-        AS[v] = leaf ? 0.f : at(kSwAS, v);
-        D[v] = leaf ? at(kSwD, v) : 0.f;
-        DB[v] = leaf ? reinterpret_cast<const double*>(st + (kSwDB * N + 2 * v) * kSwVc)[q] : 0.0;
+        const float asd = at(kSwASD, v);
+        AS[v] = leaf ? 0.f : asd;
+        D[v] = leaf ? asd : 0.f;
         UB[v] = nr ? at(kSwUB, v) : 0.f;
         GB[v] = nr ? at(kSwGB, v) : 0.f;
         AU[v] = nr ? at(kSwAU, v) : 0.f;
         BD[v] = nr ? at(kSwBD, v) : 0.f;
-        hit[v] = false;
       }
     }
     // Every value of the chunk is in registers now: stage s is free.  Order
@@ -215,8 +228,7 @@ __global__ void __launch_bounds__(kSwVc) adj_sweep_kernel(const AdjTree* __restr
             const float yv = (sw_sel(AS, p) - BD[v]) + AU[v] * icc;
             if (yv < 0.0f) continue;
             if (yv > D[v]) {
-              DB[v] += (double)SBN[v];
-              hit[v] = true;
+              atomicAdd(T.Db[v] + v0 + q, (double)SBN[v]);
               continue;
             }
             const float yb = SBN[v];
@@ -247,12 +259,7 @@ __global__ void __launch_bounds__(kSwVc) adj_sweep_kernel(const AdjTree* __restr
             const float yv = (sw_sel(AS, p) - sw_sel(BD, v)) + sw_sel(AU, v) * icc;
             if (yv < 0.0f) continue;
             if (yv > sw_sel(D, v)) {
-#pragma unroll
-              for (int w = 0; w < N; ++w)
-                if (w == v) {
-                  DB[w] += (double)sbn;
-                  hit[w] = true;
-                }
+              atomicAdd(T.Db[v] + v0 + q, (double)sbn);
               continue;
             }
             sw_add(SBO, p, sbn);
@@ -284,7 +291,6 @@ __global__ void __launch_bounds__(kSwVc) adj_sweep_kernel(const AdjTree* __restr
           S.ubo[v * arr + i] = UBO[v];
           S.dbp[v * arr + i] = DBP[v];
         }
-        if (hit[v]) T.Db[v][i] = DB[v];
       }
     }
   }

@@ -22,3 +22,11 @@ def test_window_edges(dims):
 def test_sweep_chunks_and_trees(parent, dims):
     w, truth = problem(42, dims, parent, iterations=9, smooth_nodes=(len(parent) - 1,))
     assert_matches(run_gpu(w, truth), run_oracle(w, truth), w, str((parent, dims)))
+
+
+@pytest.mark.parametrize("parent", [[1, -1], [2, 2, -1], [4, 4, 0, 0, -1], [5, 5, 0, 0, 1, -1], [6, 6, 0, 0, 1, 1, -1],
+                                    [7, 7, 7, 0, 0, 1, 1, -1], [7, 7, 7, 7, 7, 7, 7, -1], [-1, 0, 1, 2, 3, 4]])
+def test_sweep_with_the_root_last(parent):
+    """The root's place among the staged arrays; a chain."""
+    w, truth = problem(43, (20, 13, 6), parent, iterations=9, smooth_nodes=(0 if parent[0] >= 0 else 1,))
+    assert_matches(run_gpu(w, truth), run_oracle(w, truth), w, str(parent))
