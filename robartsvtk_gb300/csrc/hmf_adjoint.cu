@@ -243,7 +243,7 @@ int plan_reverse(hmf_ctx* c, cudaStream_t s) {
   for (int z = V.vz; z >= 4; --z) {
     const long long chunks = (V.vz + z - 1) / z;
     const long long waves = (per_chunk * chunks + slots - 1) / slots;
-    const double cost = (double)waves * (double)(z + 5);
+    const double cost = (double)waves * (double)(z + 6);
     if (cost < best) best = cost, best_z = z;
   }
   F.zchunk = std::min(best_z, V.vz);

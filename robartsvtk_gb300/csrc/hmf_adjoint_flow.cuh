@@ -16,12 +16,13 @@
 // the pair's other half or one warp shuffle, y neighbours go through exchange
 // rows in shared memory, z neighbours stay in registers.  Beyond the high faces
 // p', t and q are zero, so what the reference leaves out there is added as
-// zero.  Per plane k the CTA computes g,
-// p' and the total new-flow adjoint t on plane k, m / F2b and q on k-1, gb on
-// k-2 and the old-flow adjoints on k-3 (two __syncthreads per plane).  Input
-// planes arrive by cp.async.bulk.tensor into mbarrier rings two planes ahead;
-// one thread waits for them, before a barrier; every wait is bounded and a
-// time-out sets the error flag.  The plane copies are spread over the
+// zero.  The step of plane k computes g, p' and the total new-flow adjoint t on
+// plane k, m / F2b and q's x and z parts on k-1, q's y part on k-2, gb on k-3
+// and the old-flow adjoints on k-4, so that all it takes from its neighbours
+// was written before its one CTA barrier.  Input planes arrive by
+// cp.async.bulk.tensor into mbarrier rings three planes ahead; one thread waits
+// for the next step's, before the barrier; every wait is bounded and a time-out
+// sets the error flag.  The plane copies are spread over the
 // warps' first lanes (one array each, one mbarrier arrival per array), and
 // the steady planes of the march -- every stage active, no z boundary near --
 // run a copy of the step compiled without those tests.
@@ -30,7 +31,8 @@
 // rings allow (54 % of the issue slots, DRAM at 30 %).  128^3, 4 leaves: 198 us a
 // launch, against 211 us with one column and two rows per thread, scalar
 // arithmetic and the alpha gradient's sum in double (138 -> 111 million
-// instructions).
+// instructions).  With two barriers per step and a step less per chunk it took
+// 2 to 3 us more; with every thread waiting for its planes 5 us more.
 #pragma once
 
 #include <cuda.h>
@@ -49,15 +51,15 @@ constexpr int kAfMainArrays = 10;           // px, py, s, c, u, Pbx, Pby, Pbz, d
 constexpr int kAfMainSlots = 3;
 constexpr int kAfPzSlots = 4;
 // Plane k + kAfMainLead (main ring) and pz of plane k + 1 + kAfPzLead are
-// issued in step k after its first CTA barrier; the leads may rise to
-// kAfMainSlots and kAfPzSlots - 1.
-constexpr int kAfMainLead = 2;
-constexpr int kAfPzLead = 2;
+// issued in step k after its CTA barrier, when plane k has been read: the
+// leads are kAfMainSlots and kAfPzSlots - 1.
+constexpr int kAfMainLead = 3;
+constexpr int kAfPzLead = 3;
 constexpr int kAfRows = 32;                 // window rows, one per half-warp
 constexpr int kAfThreads = 16 * kAfRows;    // 512
 constexpr int kAfWarps = kAfThreads / 32;
 constexpr int kAfX = (kAfRows + 2) * 32;    // one exchange row per window row, plus zero rows -1 and 32
-constexpr int kAfXPlanes = 11;              // g, p'y[2], ty[2], m, F2b, qy[2], dbo[2]
+constexpr int kAfXPlanes = 14;              // g, p'y, ty, m, F2b, qy, dbo: two each, by step parity
 constexpr int kAfMaxOutX = 26, kAfMaxOutY = 27;
 constexpr int kAfSmemBytes =
     (kAfMainSlots * kAfMainArrays + kAfPzSlots) * kAfPlane * 4 + kAfXPlanes * kAfX * 4 + 64;
@@ -107,14 +109,14 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
   // exchange rows: *_L is read by the row above it (its y-1 neighbour), *_F by
   // the row below (y+1)
   float* XG_L = xp;
-  float* XPPY_F = xp + 1 * kAfX;  // [2] by plane parity
-  float* XTY_F = xp + 3 * kAfX;   // [2]
-  float* XM_L = xp + 5 * kAfX;
-  float* XF_L = xp + 6 * kAfX;
-  float* XQY_F = xp + 7 * kAfX;   // [2]
-  float* XD_L = xp + 9 * kAfX;    // [2]
+  float* XPPY_F = xp + 2 * kAfX;
+  float* XTY_F = xp + 4 * kAfX;
+  float* XM_L = xp + 6 * kAfX;
+  float* XF_L = xp + 8 * kAfX;
+  float* XQY_F = xp + 10 * kAfX;
+  float* XD_L = xp + 12 * kAfX;
   __shared__ int abort_cta, stall_cta;
-  __shared__ int stop;
+  __shared__ int stop_cta[2];  // by step parity
   __shared__ double red[kAfWarps];
   dependents_may_launch();
 
@@ -135,7 +137,7 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
   const int zs = item.zc * FV.zchunk;
   const int ze = min(zs + FV.zchunk, G.vz);
   const int kstart = max(zs - 3, 0);
-  const int kend = ze + 2;
+  const int kend = ze + 3;
   const int kA_end = min(ze + 1, G.vz - 1);   // last plane whose g is computed
   const int kpz_end = min(ze + 2, G.vz - 1);  // its divergence reads pz of the next plane
   const int par = fp.parity;
@@ -176,7 +178,7 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
     mbar_init(stall_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    stop = 0;
+    stop_cta[0] = stop_cta[1] = 0;
   }
   // exchange rows -1 and 32 are read as zeros (never written)
   for (int i = threadIdx.x; i < kAfXPlanes * kAfX; i += kAfThreads) xp[i] = 0.f;
@@ -201,20 +203,22 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
     mbar_expect_tx(bar, (unsigned)(kAfBoxX * kAfBoxY * 4));
     tma_load_plane(zslot(p), &V->pz, xs, y0 - 3, p, bar);
   };
-  // Thread 0 alone waits for the planes a step reads, just before a CTA
-  // barrier that precedes the reads (the barrier extends its acquire to every
-  // thread).  A wait that runs out raises `stop`, read by all after the
-  // barrier: the CTA leaves the march, drains its copies and reports.
-  auto wait0 = [&](uint64_t* bar, unsigned parity) {  // thread 0 only
-    if (stop) return;
-    if (!mbar_wait_bounded(bar, parity, fp.wait_limit_ns)) stop = 1;
+  // Thread 0 alone waits for the planes the next step reads, before the step's
+  // CTA barrier (the barrier extends its acquire to every thread).  A wait that
+  // runs out raises the step's flag, read by all after its barrier: the CTA
+  // leaves the march, drains its copies and reports.
+  bool timed_out = false;
+  auto wait0 = [&](uint64_t* bar, unsigned parity, int k) {  // thread 0 only
+    if (timed_out || mbar_wait_bounded(bar, parity, fp.wait_limit_ns)) return;
+    timed_out = true;
+    *(volatile int*)&stop_cta[k & 1] = 1;
   };
   int k_stop = -1;  // the step at which the march stopped (-1: it ran to the end)
-  auto wait_main0 = [&](int p) {
-    wait0(&mbars[(p - kstart) % kAfMainSlots], (unsigned)(((p - kstart) / kAfMainSlots) & 1));
+  auto wait_main0 = [&](int p, int k) {
+    wait0(&mbars[(p - kstart) % kAfMainSlots], (unsigned)(((p - kstart) / kAfMainSlots) & 1), k);
   };
-  auto wait_pz0 = [&](int p) {
-    wait0(&zbars[(p - kstart) % kAfPzSlots], (unsigned)(((p - kstart) / kAfPzSlots) & 1));
+  auto wait_pz0 = [&](int p, int k) {
+    wait0(&zbars[(p - kstart) % kAfPzSlots], (unsigned)(((p - kstart) / kAfPzSlots) & 1), k);
   };
   // Lane 0 of warp a issues every copy of main-ring array a, lane 0 of the
   // last warp every z-flow copy; each first acquires the one map it uses.
@@ -229,11 +233,11 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
     }
   }
   if (threadIdx.x == 0) {
-    wait_main0(kstart);
-    wait_pz0(kstart);
-    if (kstart + 1 < G.vz) wait_pz0(kstart + 1);
+    wait_main0(kstart, kstart);
+    wait_pz0(kstart, kstart);
+    if (kstart + 1 < G.vz) wait_pz0(kstart + 1, kstart);
     // the failure path on demand: a wait on a barrier that no copy completes
-    if (stall_cta) wait0(stall_bar, 0);
+    if (stall_cta) wait0(stall_bar, 0, kstart);
   }
   __syncthreads();
 
@@ -257,16 +261,17 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
     F2 gprev = zero2, dbp_prev = zero2;                                                              // plane k-1
     F2 ppx = zero2, ppy = zero2, ppz = zero2, tx = zero2, ty = zero2, tz = zero2, S_c = zero2;       // k-1
     F2 m_prev = f2(1.0f), f_prev = zero2;                                                            // k-2
-    F2 qx_e = zero2, qy_e = zero2, qz_e = zero2;                                                     // q of k-2
-    F2 qx_f = zero2, qy_f = zero2, qz_f = zero2;                                                     // q of k-3
-    F2 dbo_f = zero2, dbo_ff = zero2;                                                                // k-3, k-4
+    F2 qx_d = zero2, qz_d = zero2;                                                                   // q of k-2
+    F2 qx_e = zero2, qy_e = zero2, qz_e = zero2;                                                     // q of k-3
+    F2 qx_f = zero2, qy_f = zero2, qz_f = zero2;                                                     // q of k-4
+    F2 dbo_f = zero2, dbo_ff = zero2;                                                                // k-4, k-5
     F2 pzn_c = zero2;
     bool have_pz = false;
     const float* cur = mslot(kstart);
     const float* zc = zslot(kstart);
     int msi = 0, zsi = 0;                           // ring positions of plane k
-    long long go = (long long)(kstart - 2) * G.plane;  // plane offset of gb outputs (plane k-2)
-    long long fo = (long long)(kstart - 3) * G.plane;  // ... of old-flow outputs (plane k-3)
+    long long go = (long long)(kstart - 3) * G.plane;  // plane offset of gb outputs (plane k-3)
+    long long fo = (long long)(kstart - 4) * G.plane;  // ... of old-flow outputs (plane k-4)
 
     // returns false when the march stops (a copy wait ran out)
     auto zstep = [&](const int k, auto stag) -> bool {
@@ -274,11 +279,12 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
       const bool doA = ST || k <= kA_end;
       const int kc = k - 1;
       const bool doC = ST || (kc >= kstart && kc <= min(ze, G.vz - 1));
-      const int ko = k - 2;
+      const bool doY = ST || (k - 2 >= kstart && k - 2 <= min(ze, G.vz - 1));
+      const int ko = k - 3;
       const bool doE = ST || (ko >= kstart && ko <= ze - 1);
-      const int kf = k - 3;
+      const int kf = k - 4;
       const bool doF = ST || (kf >= zs && kf < ze);
-      const int kb = k & 1;  // exchange-row parity of plane k
+      const int now = (k & 1) * kAfX + xw, before = ((k & 1) ^ 1) * kAfX + xw;  // exchange rows of this step, of the last
 
       // ---- stage A: g(k) (kern_CalcGradStep on the recomputed divergence)
       F2 g = zero2, px = zero2, py = zero2, pz = zero2, Pbx = zero2, Pby = zero2, Pbz = zero2, dbp = zero2,
@@ -310,8 +316,16 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
         pzn_c = pzn;
         have_pz = has_next;
       }
-      f2_st(XG_L + xw, g);
-      __syncthreads();  // (1)
+      f2_st(XG_L + now, g);
+      if (threadIdx.x == 0) {  // the planes the next step's stage A reads
+        if (k + 1 <= kA_end) wait_main0(k + 1, k);
+        if (k + 2 < G.vz && k + 2 <= kpz_end) wait_pz0(k + 2, k);
+      }
+      __syncthreads();
+      if (*(volatile int*)&stop_cta[k & 1]) {
+        k_stop = k;
+        return false;
+      }
       if (lane == 0) {
         if (warp < narr && k + kAfMainLead <= kA_end) issue_main_array(k + kAfMainLead, warp, warp_map);
         if (warp == kAfWarps - 1 && k + 1 + kAfPzLead <= kpz_end) issue_pz(k + 1 + kAfPzLead);
@@ -320,7 +334,7 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
       // ---- stage B: p'(k) (kern_DescentSpatialFlow) and the total adjoint t(k)
       // of the new flows (incoming plus through the new divergence)
       F2 ppx_n = off_x(px - (g - left(g)));
-      F2 ppy_n = off_y(py - (g - f2_ld(XG_L + xw - 32)));
+      F2 ppy_n = off_y(py - (g - f2_ld(XG_L + now - 32)));
       F2 ppz_n = inside(pz - (g - gprev));
       F2 tx_n = inside((Pbx + dbp) - dbpl);
       F2 ty_n = inside((Pby + dbp) - dbpu);
@@ -333,14 +347,15 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
         gprev = g;
         dbp_prev = dbp;
       }
-      f2_st(XPPY_F + kb * kAfX + xw, ppy_n);
-      f2_st(XTY_F + kb * kAfX + xw, ty_n);
+      const F2 ppy_2 = f2_ld(XPPY_F + now), ty_2 = f2_ld(XTY_F + now);  // this thread's of plane k-2
+      f2_st(XPPY_F + now, ppy_n);
+      f2_st(XTY_F + now, ty_n);
 
       // ---- stage C: |p|, m(k-1) and the adjoint of the multiplier -> F2b(k-1)
       F2 m = f2(1.0f), f2b = zero2;
       {
-        const F2 pyd = f2_ld(XPPY_F + (kb ^ 1) * kAfX + xw + 32);
-        const F2 tyd = f2_ld(XTY_F + (kb ^ 1) * kAfX + xw + 32);
+        const F2 pyd = f2_ld(XPPY_F + before + 32);
+        const F2 tyd = f2_ld(XTY_F + before + 32);
         const F2 pxr = right(ppx), txr = right(tx);
         F2 f = mul(ppx, ppx) + mul(pxr, pxr);
         f = f + (mul(ppy, ppy) + mul(pyd, pyd));
@@ -383,50 +398,45 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
           m = f2(mv[0], mv[1]);
           f2b = f2(fv[0], fv[1]);
         }
-        f2_st(XM_L + xw, m);
-        f2_st(XF_L + xw, f2b);
-      }
-      if (threadIdx.x == 0) {  // the planes the next step's stage A reads
-        if (k + 1 <= kA_end) wait_main0(k + 1);
-        if (k + 2 < G.vz && k + 2 <= kpz_end) wait_pz0(k + 2);
-      }
-      __syncthreads();  // (2)
-      if (stop) {
-        k_stop = k;
-        return false;
+        f2_st(XM_L + now, m);
+        f2_st(XF_L + now, f2b);
       }
 
-      // ---- stage D: q(k-1), the adjoint of p'
-      F2 qx_n = zero2, qy_n = zero2, qz_n = zero2;
+      // ---- stage D: q, the adjoint of p': the x and z parts of plane k-1; the
+      // y part, which takes the row above's m, of plane k-2
+      F2 qy_n = zero2;
+      if (doY) {
+        const F2 mup = f2_ld(XM_L + before - 32), fup = f2_ld(XF_L + before - 32);
+        qy_n = off_y(mul(mul(ty_2, half2), m_prev + mup) + mul(mul(two2, ppy_2), f_prev + fup));
+      }
+      F2 qx_n = zero2, qz_n = zero2;
       if (doC) {
-        const F2 mup = f2_ld(XM_L + xw - 32), fup = f2_ld(XF_L + xw - 32);
         qx_n = off_x(mul(mul(tx, half2), m + left(m)) + mul(mul(two2, ppx), f2b + left(f2b)));
-        qy_n = off_y(mul(mul(ty, half2), m + mup) + mul(mul(two2, ppy), f2b + fup));
         if (ST || kc > 0) qz_n = inside(mul(mul(tz, half2), m + m_prev) + mul(mul(two2, ppz), f2b + f_prev));
         m_prev = m;
         f_prev = f2b;
       }
-      f2_st(XQY_F + (kb ^ 1) * kAfX + xw, qy_n);  // plane k-1
+      f2_st(XQY_F + now, qy_n);  // plane k-2
 
-      // ---- stage E: gb(k-2), the adjoint of g, and dbo = step * gb
+      // ---- stage E: gb(k-3), the adjoint of g, and dbo = step * gb
       F2 dbo = zero2;
       {
-        const F2 qyd = f2_ld(XQY_F + kb * kAfX + xw + 32);  // plane k-2
+        const F2 qyd = f2_ld(XQY_F + before + 32);  // plane k-3
         const F2 s3 = (qx_e + qy_e) + qz_e;
         F2 gb = f2(-f2_lo(s3), -f2_hi(s3));
         gb = gb + right(qx_e);
         gb = gb + qyd;
-        gb = gb + qz_n;
+        gb = gb + qz_d;
         if (doE) {
           dbo = inside(mul(step2, gb));
           if (own && (ST || ko >= zs)) f2_st(ogb + (go + rowoff), inside(gb));
         }
-        f2_st(XD_L + kb * kAfX + xw, dbo);  // plane k-2
+        f2_st(XD_L + now, dbo);  // plane k-3
       }
 
-      // ---- stage F: adjoint of the old flows at k-3
+      // ---- stage F: adjoint of the old flows at k-4
       {
-        const F2 dup = f2_ld(XD_L + (kb ^ 1) * kAfX + xw - 32);  // plane k-3
+        const F2 dup = f2_ld(XD_L + before - 32);  // plane k-4
         const F2 dxl = left(dbo_f);
         if (doF && own) {
           const long long o = fo + rowoff;
@@ -447,9 +457,11 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
       qx_f = qx_e;
       qy_f = qy_e;
       qz_f = qz_e;
-      qx_e = qx_n;
+      qx_e = qx_d;
       qy_e = qy_n;
-      qz_e = qz_n;
+      qz_e = qz_d;
+      qx_d = qx_n;
+      qz_d = qz_n;
       dbo_ff = dbo_f;
       dbo_f = dbo;
       msi = msi + 1 == kAfMainSlots ? 0 : msi + 1;
@@ -460,7 +472,7 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
       fo += G.plane;
       return true;
     };
-    const int k_lo = zs + 4, k_hi = min(ze + 1, G.vz - 2);
+    const int k_lo = zs + 5, k_hi = min(ze + 1, G.vz - 2);
     int k = kstart;
     bool go_on = true;
     for (; go_on && k <= kend && k < k_lo; ++k) go_on = zstep(k, BoolTag<false>{});
@@ -469,7 +481,6 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
   };
   if (interior) march(BoolTag<true>{});
   else march(BoolTag<false>{});
-  const bool timed_out = stop != 0;
 
   // alpha gradient: block sum, one atomic per CTA
   double alpha_sum = (double)asum.hi + (double)asum.lo;
@@ -484,12 +495,12 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
   if (timed_out && threadIdx.x == 0) {
     if (fp.error_flag) atomicOr(fp.error_flag, 2);
     // Copies still in flight into this CTA's shared memory must land before
-    // it exits.  Up to step k_stop the main ring was filled to plane
-    // k_stop + kAfMainLead and the pz ring to k_stop + 1 + kAfPzLead (the
+    // it exits.  Up to the step before k_stop, ks, the main ring was filled to
+    // plane ks + kAfMainLead and the pz ring to ks + 1 + kAfPzLead (the
     // initial issue: kstart - 1 + kAfMainLead, kstart + kAfPzLead), each slot
     // holding at most one pending phase: wait for the last plane issued into
     // each slot, with the default bound.
-    const int ks = k_stop >= 0 ? k_stop : kstart;
+    const int ks = max(k_stop, kstart) - 1;
     const int l_main = min(max(ks + kAfMainLead, kstart + kAfMainLead - 1), kA_end);
     const int l_pz = min(max(ks + 1 + kAfPzLead, kstart + kAfPzLead), kpz_end);
     for (int p = max(kstart, l_main - kAfMainSlots + 1); p <= l_main; ++p)
