@@ -255,15 +255,17 @@ int hmf_get_flow_window(const hmf_ctx* ctx);
  * 1, 2 and 4 with its best window and chunk.  Results do not depend on it. */
 int hmf_set_flow_units(hmf_ctx* ctx, int units);
 int hmf_get_flow_units(const hmf_ctx* ctx);
-/* Slab pipeline of the replayed iterations (single volumes of label trees,
- * REF_CUDA, convergence log off): each iteration's flow and sweep launches
- * are cut at the flow plan's z chunks into per-slab graph nodes that wait
- * only for the slabs their stencil touches, so sweeps overlap flows and
- * consecutive iterations overlap.  Same arithmetic, bit-identical results.
- * On by default; hmf_get_pipeline returns 1 when it is on and the plan allows
- * it.  On the default plan a volume small enough for the whole flow step to be
- * resident at once runs in whole launches all the same (a z chunk, window or
- * units per CTA set by the caller are pipelined at any size). */
+/* Slab pipeline of the replayed iterations (single volumes of label trees, and
+ * of graphs of up to 8 nodes without repeated edges; REF_CUDA): each
+ * iteration's flow and sweep launches are cut at the flow plan's z chunks into
+ * per-slab graph nodes that wait only for the slabs their stencil touches, so
+ * sweeps overlap flows and consecutive iterations overlap.  Same arithmetic,
+ * bit-identical results.  On by default; hmf_get_pipeline returns 1 when it is
+ * on and a label tree's plan allows it.  On the default plan a volume whose
+ * flow step is resident on the GPU at once runs in whole launches all the same,
+ * and one of at most 350,000 voxel-vertices in kernels of its own that no plan
+ * concerns (a z chunk, window or units per CTA set by the caller are pipelined
+ * at any size). */
 int hmf_set_pipeline(hmf_ctx* ctx, int enabled);
 int hmf_get_pipeline(const hmf_ctx* ctx);
 
