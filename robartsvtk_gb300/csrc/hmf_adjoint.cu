@@ -221,10 +221,10 @@ float* pb_array(const AdjointState* S, const hmf_ctx* c, int parity, int v, int 
   return axis == 0 ? c->fx[1][v] : axis == 1 ? c->fy[1][v] : c->fz[1][v];  // null for the root (no flows)
 }
 
-// Windows of at most 27 x 27 outputs spread evenly over the volume; z chunk:
-// the one that minimises waves x planes marched per CTA, with one CTA per SM
-// and the five halo planes the reverse chain reaches (3 low, 2 high) -- the
-// work of a wave is set by its longest CTA, so a last, partial wave costs as
+// Windows of at most 26 x 27 outputs spread evenly over the volume; z chunk:
+// the one that minimises waves x steps per CTA, with one CTA per SM, the five
+// halo planes the reverse chain reaches (3 low, 2 high) and the step its last
+// stage lags -- the work of a wave is set by its longest CTA, so a last, partial wave costs as
 // much as a full one.
 int plan_reverse(hmf_ctx* c, cudaStream_t s) {
   AdjointState* S = c->adj;

@@ -28,11 +28,11 @@
 // run a copy of the step compiled without those tests.
 //
 // What bounds it: latency and issue with the 16 warps that its registers and
-// rings allow (54 % of the issue slots, DRAM at 30 %).  128^3, 4 leaves: 198 us a
-// launch, against 211 us with one column and two rows per thread, scalar
-// arithmetic and the alpha gradient's sum in double (138 -> 111 million
-// instructions).  With two barriers per step and a step less per chunk it took
-// 2 to 3 us more; with every thread waiting for its planes 5 us more.
+// rings allow (63 % of the issue slots, DRAM at 31 %).  128^3, 4 leaves, the mean of
+// 300 steps: 196 us a launch, against 211 us with one column and two rows per
+// thread, scalar arithmetic and the alpha gradient's sum in double.  With two
+// barriers per step and a step less per chunk it took 2 to 3 us more (54 % of
+// the issue slots); with every thread waiting for its planes 5 us more.
 #pragma once
 
 #include <cuda.h>
