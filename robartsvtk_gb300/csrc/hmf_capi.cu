@@ -362,6 +362,14 @@ int plan_flow(hmf_ctx* c, int zchunk) {
 // 0.93: 144.4 us whole, 126.0 in five slabs; 110^3 four leaves, 1.05: 96.1
 // and 91.7; 84 x 80 x 190 tree5, 1.11: 107.9 and 111.3; 168 x 162 x 62 four
 // leaves, 1.21: 90.9 and 95.9).
+//
+// A pipelined batch has no waves (its groups' launches overlap): what counts is
+// the planes marched and, a little, the longest march, with which a group's
+// iteration ends.  Per iteration, three leaves, chunks by waves and by this rule:
+// 20 volumes of 48..192 (37 and 93 planes) 1316 and 1268 us, 10 of 64..176 (29
+// and 86) 689 and 632, 6 of 30..150 (21 and 36) 138 and 126, 4 of 60..170 (24 and
+// 48) 215 and 201, 60 of 20..60 (30 and 60) 219 and 206, 3 of 200..280 (four
+// leaves, 37 and 85) 833 and 836.
 int default_zchunk(const hmf_ctx* c) {
   const int oy = flow_max_out_y(c);
   const long long slots = flow_slots(c);
@@ -375,7 +383,8 @@ int default_zchunk(const hmf_ctx* c) {
   // a wave covers about one row of windows only when one volume's chunk
   // takes many waves (a batch of small volumes puts whole volumes in a wave)
   const bool pipelined = c->pipeline && c->vols.size() == 1 && (!c->dag || c->n <= hmf::kDagRegMax);
-  const int cap = per_chunk > 8 * slots ? 24 : (pipelined ? 64 : 48);
+  const bool batched = c->pipeline && c->vols.size() > 1;
+  const int cap = per_chunk > 8 * slots ? 24 : batched ? 96 : pipelined ? 64 : 48;
   const int third = (maxz + 2) / 3;
   const bool slabs = pipelined && third >= 20;
   const int slab_cap = slabs ? third : cap;  // of plans of more than one wave
@@ -384,15 +393,18 @@ int default_zchunk(const hmf_ctx* c) {
   for (int chunks = 1; chunks <= maxz; ++chunks) {
     const int z = (maxz + chunks - 1) / chunks;
     if (z > cap) continue;
-    long long ctas = 0;
+    long long ctas = 0, planes = 0;  // CTAs, and the planes they march
     for (const auto& V : c->vols) {
-      const int zv = std::min(z, V.vz);
-      ctas += (long long)((V.vx + hmf::kTmaMaxOutX - 1) / hmf::kTmaMaxOutX) *
-              ((V.vy + oy - 1) / oy) * ((V.vz + zv - 1) / zv) * (c->n - 1);
+      const int zv = std::min(z, V.vz), n = (V.vz + zv - 1) / zv;
+      const long long windows =
+          (long long)((V.vx + hmf::kTmaMaxOutX - 1) / hmf::kTmaMaxOutX) * ((V.vy + oy - 1) / oy) * (c->n - 1);
+      ctas += windows * n;
+      planes += windows * (V.vz + 6LL * n);
     }
     if (z > slab_cap && ctas > slots) continue;
     double cost = (double)((ctas + slots - 1) / slots) * (double)(z + 7);
     if (slabs && ctas > slots) cost *= 0.9;
+    if (batched) cost = (double)planes / (double)slots + 0.2 * (double)(z + 7);
     if (cost < best) best = cost, best_z = z;  // ties keep the longer chunk
   }
   return best_z;

@@ -8,6 +8,7 @@ import pytest
 
 from robartsvtk_gb300 import DAGSolver, HMFSolver
 from robartsvtk_gb300.synthetic import random_tree_problem
+from tests.test_gpu_batch import make_batch, solve_batch
 from tests.test_gpu_dag import assert_exact, oracle_solve, random_dag
 from tests.test_gpu_parity import assert_same, oracle, run_gpu
 
@@ -92,3 +93,14 @@ def test_graph_in_slabs(dims, zchunk, iterations, slabs):
             assert_exact({"u": {v: s.labels(v) for v in range(1, w.n)}, "sink": {v: s.sink(v) for v in range(w.n)}}, o,
                          str(dims))
             assert s.stats()["launches"] == 1 + 2 * slabs * (iterations - 1) + 2
+
+
+@pytest.mark.parametrize("dims", [
+    [(40, 33, 100), (30, 41, 61), (57, 28, 35), (29, 27, 3)] * 3,  # one long chunk for some, several for others
+    [(20, 18, 70), (9, 40, 33)],                                   # few windows: short chunks
+])
+def test_batch_default_plan(dims):
+    ws = make_batch(21, dims, parent=[-1, 0, 0, 1, 1], iterations=3, smooth_nodes=(1,))
+    got, _ = solve_batch(ws)
+    for i, w in enumerate(ws):
+        assert_same(got[i], oracle(w), "volume %d %s" % (i, w.dims))
