@@ -1867,7 +1867,8 @@ int hmf_autotune(hmf_ctx* c, void* stream) {
   const bool saved_timing = c->timing;
   int maxz = 1;
   for (const auto& V : c->vols) maxz = std::max(maxz, V.vz);
-  TunedPlan best{c->flow_warps, c->zchunk, c->flow_units};
+  const TunedPlan before{c->flow_warps, c->zchunk, c->flow_units};
+  TunedPlan best = before;
   double best_ms = 1e30;
   int rc = HMF_OK;
   DeviceGuard dg(c->device);
@@ -1939,12 +1940,16 @@ int hmf_autotune(hmf_ctx* c, void* stream) {
   c->timing = saved_timing;
   c->tuning = false;
   c->solved = false;
-  c->flow_warps = best.warps;
-  c->flow_units = best.units;
-  if (rc) return rc;
+  // After a failure too the context leaves with one plan, its own of before, and
+  // without the last candidate's graphs: the next solve may run other kernels,
+  // which do not rewrite the tables that those graphs read.
+  const TunedPlan& keep = rc ? before : best;
   drop_graphs(c);
-  rc = plan_flow(c, best.zchunk);
+  c->flow_warps = keep.warps;
+  c->flow_units = keep.units;
+  const int planned = plan_flow(c, keep.zchunk);
   if (rc) return rc;
+  if (planned) return planned;
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   const std::string key = tune_key(c);
   g_tune_cache[key] = best;

@@ -1,0 +1,47 @@
+"""Which kernels and launches a solve takes, and what the calls that choose them
+promise: settings that the caller made stay in force, the pipeline's getter says
+how the next solve runs, and a failed autotune changes nothing.  Results are the
+oracle's bit for bit on every route.  GPU only."""
+import numpy as np
+import pytest
+
+from robartsvtk_gb300 import HMFError, HMFSolver
+from robartsvtk_gb300.synthetic import random_tree_problem
+from tests.test_gpu_parity import oracle
+
+pytestmark = pytest.mark.gpu
+
+TREE5 = [-1, 0, 0, 1, 1]
+
+
+def fill(s, w):
+    for leaf, d in w.data.items():
+        s.set_data(leaf, d)
+    for v, S in w.smooth.items():
+        s.set_smoothness(v, S)
+    for v, a in w.alpha.items():
+        s.set_smoothness_scalar(v, a)
+    s.set_params(w.iterations, w.step, w.cc)
+
+
+def assert_oracle(s, w, what=""):
+    ref = oracle(w)
+    for v in range(len(w.parent)):
+        assert np.array_equal(s.sink(v), ref["sink"][v].astype(np.float32)), (what, v)
+        if w.parent[v] >= 0:
+            assert np.array_equal(s.labels(v), ref["u"][v].astype(np.float32)), (what, v)
+
+
+@pytest.mark.parametrize("dims", [(40, 36, 28), (90, 75, 33)])
+def test_failed_autotune_leaves_the_plan(dims):
+    w = random_tree_problem(27, dims, TREE5, iterations=7, smooth_nodes=(1,))
+    with HMFSolver(w.dims, w.parent) as s:
+        s.set_flow_window(64)
+        s.set_zchunk(5)
+        s.set_flow_units(2)
+        with pytest.raises(HMFError, match="[Mm]issing data"):
+            s.autotune()
+        assert (s.flow_window, s.zchunk(), s.flow_units) == (64, 5, 2)
+        fill(s, w)
+        s.solve()
+        assert_oracle(s, w, dims)
