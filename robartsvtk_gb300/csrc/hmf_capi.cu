@@ -591,8 +591,11 @@ int launch_flow_tma_items(hmf_ctx* c, const hmf::FlowVertexTMA* table, int parit
 // -- 389,000 -- 24.8 against 23.9, 64^3 35.9 against 31.3).
 constexpr long long kCellVoxels = 350000;
 
+// No part of the march's plan was chosen by the caller.
+bool default_flow(const hmf_ctx* c) { return !c->window_set && !c->zchunk_set && !c->units_set; }
+
 bool cell_path(const hmf_ctx* c) {
-  return c->default_flow && !c->tuning && c->pipeline && c->use_tma && c->tree_kind == 0 && !c->dag && c->vols.size() == 1 &&
+  return default_flow(c) && !c->tuning && c->pipeline && c->use_tma && c->tree_kind == 0 && !c->dag && c->vols.size() == 1 &&
          c->n <= hmf::kSweepCellMax && !c->gap_on && c->stall_kind < 0 && c->semantics == HMF_SEMANTICS_REF_CUDA &&
          c->total * (c->n - 1) <= kCellVoxels;
 }
@@ -875,7 +878,7 @@ bool pipeline_active(const hmf_ctx* c) { return !c->dag && slabs_possible(c); }
 // leaves: 157.1 against 175.6).
 bool slab_replay(const hmf_ctx* c) {
   if (!slabs_possible(c) || cell_path(c)) return false;
-  if (!c->default_flow || c->vols.size() > 1) return true;
+  if (!default_flow(c) || c->vols.size() > 1) return true;
   const long long units = (long long)c->n_items * (c->n - 1);
   return (units + c->flow_units - 1) / c->flow_units > flow_slots(c);
 }
@@ -1977,7 +1980,8 @@ int hmf_set_flow_window(hmf_ctx* c, int rows) {
   DeviceGuard dg(c->device);
   drop_graphs(c);
   c->flow_warps = rows == 64 ? 16 : 8;
-  c->default_flow = rows == 0;
+  c->window_set = rows != 0;
+  c->zchunk_set = false;  // planned again
   return plan_flow(c, default_zchunk(c));
 }
 
@@ -1991,7 +1995,7 @@ int hmf_set_flow_units(hmf_ctx* c, int units) {
   DeviceGuard dg(c->device);
   drop_graphs(c);  // the captured launches carry the grid
   c->flow_units = units ? units : 1;
-  c->default_flow = units == 0;
+  c->units_set = units != 0;
   return HMF_OK;
 }
 
@@ -2005,7 +2009,7 @@ int hmf_set_zchunk(hmf_ctx* c, int z) {
   drop_graphs(c);
   int maxz = 1;
   for (const auto& V : c->vols) maxz = std::max(maxz, V.vz);
-  c->default_flow = z == 0;
+  c->zchunk_set = z != 0;
   return plan_flow(c, z ? std::min(z, maxz) : default_zchunk(c));
 }
 

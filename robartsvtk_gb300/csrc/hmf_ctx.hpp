@@ -69,7 +69,7 @@ struct hmf_ctx {
   int n_items = 0;
   int zchunk = 0;  // planes per window column (0: not planned yet)
   int flow_warps = 8;  // flow_tma_kernel<W>: windows of 32 x 4W (hmf_set_flow_window)
-  bool default_flow = true;  // no window, z chunk or units set by the caller (hmf_cell.cuh may run)
+  bool window_set = false, zchunk_set = false, units_set = false;  // chosen by the caller, each until set to 0
   bool tuning = false;        // hmf_autotune times the march's plans
   bool overlap_launches = false;  // launches now recorded let the next kernel start early (launch_waiting)
   int flow_units = 1;  // flow_tma_kernel: (window, vertex) units marched by one CTA (hmf_set_flow_units)

@@ -45,3 +45,42 @@ def test_failed_autotune_leaves_the_plan(dims):
         fill(s, w)
         s.solve()
         assert_oracle(s, w, dims)
+
+
+@pytest.mark.parametrize("calls", [
+    [("zchunk", 5), ("units", 0)],
+    [("zchunk", 5), ("units", 4), ("units", 0)],
+    [("units", 2), ("zchunk", 5), ("zchunk", 0)],
+    [("window", 64), ("units", 0)],
+    [("window", 64), ("zchunk", 0)],
+    [("window", 32), ("zchunk", 5), ("zchunk", 0)],
+])
+def test_a_setting_stays_until_it_is_set_to_zero(calls):
+    """A plan of the caller's is pipelined at any size, whatever other setting
+    is restored after it; with every setting restored the default plan runs."""
+    w = random_tree_problem(28, (40, 30, 60), TREE5, iterations=6, smooth_nodes=(1,))  # default chunks of 3 planes or more
+    with HMFSolver(w.dims, w.parent) as s:
+        setters = {"zchunk": s.set_zchunk, "units": s.set_flow_units, "window": s.set_flow_window}
+        for name, value in calls:
+            setters[name](value)
+        fill(s, w)
+        s.solve()
+        slabs = -(-w.dims[2] // s.zchunk())
+        assert slabs > 1 and s.stats()["launches"] == 1 + 2 * slabs * w.iterations
+        assert_oracle(s, w, calls)
+        for name in ("window", "zchunk", "units"):
+            setters[name](0)
+        s.solve()
+        assert s.stats()["launches"] == 1 + 2 * w.iterations
+        assert_oracle(s, w, calls)
+
+
+def test_a_window_restores_the_default_chunk():
+    with HMFSolver((40, 30, 20), TREE5) as s:
+        z = s.zchunk()
+        s.set_zchunk(5)
+        s.set_flow_window(0)
+        w = random_tree_problem(28, (40, 30, 20), TREE5, iterations=6)
+        fill(s, w)
+        s.solve()
+        assert s.zchunk() == z and s.stats()["launches"] == 1 + 2 * w.iterations
