@@ -233,7 +233,9 @@ int hmf_batch_get_sink(hmf_ctx* ctx, int volume, int node, float* out, int where
  * 4 units per CTA (hmf_set_flow_units), on the context's current inputs,
  * keeps the fastest for this context and caches it for contexts of the same
  * shape created later (key: SM count, semantics, tree shape, volume sizes
- * rounded up to multiples of 16).  The cache lives for the process; with the
+ * rounded up to multiples of 16).  A volume small enough for the kernels of
+ * its own (hmf_set_pipeline) is timed with them first; they stay unless a plan
+ * is faster, and such volumes are cached apart.  The cache lives for the process; with the
  * environment variable HMF_AUTOTUNE_CACHE naming a file it is also read from
  * and appended to that file.  Inputs must be set; the labels are not kept. */
 int hmf_autotune(hmf_ctx* ctx, void* stream);

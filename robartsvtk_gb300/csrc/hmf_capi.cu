@@ -594,10 +594,15 @@ constexpr long long kCellVoxels = 350000;
 // No part of the march's plan was chosen by the caller.
 bool default_flow(const hmf_ctx* c) { return !c->window_set && !c->zchunk_set && !c->units_set; }
 
+// What the context is, whatever was set on it since.
+bool cells_possible(const hmf_ctx* c) {
+  return c->use_tma && c->tree_kind == 0 && !c->dag && c->vols.size() == 1 && c->n <= hmf::kSweepCellMax &&
+         c->semantics == HMF_SEMANTICS_REF_CUDA && c->total * (c->n - 1) <= kCellVoxels;
+}
+
 bool cell_path(const hmf_ctx* c) {
-  return default_flow(c) && !c->tuning && c->pipeline && c->use_tma && c->tree_kind == 0 && !c->dag && c->vols.size() == 1 &&
-         c->n <= hmf::kSweepCellMax && !c->gap_on && c->stall_kind < 0 && c->semantics == HMF_SEMANTICS_REF_CUDA &&
-         c->total * (c->n - 1) <= kCellVoxels;
+  return cells_possible(c) && default_flow(c) && !c->march_tuned && !c->tuning && c->pipeline && !c->gap_on &&
+         c->stall_kind < 0;
 }
 
 int launch_flow_cell(hmf_ctx* c, int parity, cudaStream_t s) {
@@ -1391,7 +1396,9 @@ int copy_out(hmf_ctx* c, int b, const float* src, float* out, int where, void* s
 // to a multiple of 16 (sizes in one bucket share window counts within one
 // and the same z-chunk choices).  Process-wide; with HMF_AUTOTUNE_CACHE set
 // to a file path it is also read from and appended to that file (one
-// "key warps zchunk" line per tuned shape), so later processes reuse it.
+// "key warps zchunk units" line per tuned shape), so later processes reuse it.
+// Where the cell kernels could run the key says so: only there was the march
+// timed against them, and units 0 says that they won (on the default plan).
 struct TunedPlan {
   int warps, zchunk, units;
 };
@@ -1399,8 +1406,8 @@ std::mutex g_tune_mutex;
 std::map<std::string, TunedPlan> g_tune_cache;
 bool g_tune_file_read = false;
 
-std::string tune_key(const hmf_ctx* c) {
-  std::string k = std::to_string(c->sm_count) + "/" + std::to_string(c->semantics) + "/n" + std::to_string(c->n) + ":";
+std::string tune_key(const hmf_ctx* c, bool cells) {
+  std::string k = (cells ? "cells/" : "") + std::to_string(c->sm_count) + "/" + std::to_string(c->semantics) + "/n" + std::to_string(c->n) + ":";
   for (int v : c->preorder) k += std::to_string(c->kids[v].size()) + ",";
   for (const auto& V : c->vols)
     k += "/" + std::to_string((V.vx + 15) / 16 * 16) + "x" + std::to_string((V.vy + 15) / 16 * 16) + "x" +
@@ -1419,7 +1426,7 @@ void tune_file_read() {
   char line[4200], key[4096];
   while (std::fgets(line, sizeof(line), f)) {
     int w = 0, z = 0, u = 1;  // lines written before the units field read as one unit per CTA
-    if (std::sscanf(line, "%4095s %d %d %d", key, &w, &z, &u) >= 3 && (w == 8 || w == 16) && z >= 1 && u >= 1 &&
+    if (std::sscanf(line, "%4095s %d %d %d", key, &w, &z, &u) >= 3 && (w == 8 || w == 16) && z >= 1 && u >= 0 &&
         u <= kMaxFlowUnits)
       g_tune_cache[key] = TunedPlan{w, z, u};
   }
@@ -1586,11 +1593,12 @@ int create_context(hmf_ctx** out, int n_volumes, const int* dims, int semantics,
       {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         tune_file_read();
-        auto it = g_tune_cache.find(tune_key(c));
-        if (it != g_tune_cache.end()) {
+        auto it = g_tune_cache.find(tune_key(c, cells_possible(c)));
+        if (it != g_tune_cache.end() && it->second.units > 0) {
           c->flow_warps = it->second.warps;
           c->flow_units = it->second.units;
           z = it->second.zchunk;
+          c->march_tuned = true;
         }
       }
       rc = plan_flow(c, z ? z : default_zchunk(c));
@@ -1871,6 +1879,9 @@ int hmf_autotune(hmf_ctx* c, void* stream) {
   int maxz = 1;
   for (const auto& V : c->vols) maxz = std::max(maxz, V.vz);
   const TunedPlan before{c->flow_warps, c->zchunk, c->flow_units};
+  const bool saved_tuned = c->march_tuned;
+  c->march_tuned = false;
+  const bool cells = cell_path(c);  // what the context runs unless a plan of the march is faster
   TunedPlan best = before;
   double best_ms = 1e30;
   int rc = HMF_OK;
@@ -1885,15 +1896,15 @@ int hmf_autotune(hmf_ctx* c, void* stream) {
   // default plan is timed first).  Candidates, for each window shape
   // (32 x 32 and 32 x 64): the default plan's chunk, then 16, 24, 32, 48, 64,
   // 96, ... up to the longest volume, one unit per CTA; then the best of
-  // those with 2 and 4 units (window-vertex marches) per CTA.
+  // those with 2 and 4 units (window-vertex marches) per CTA.  A volume that the
+  // cell kernels take is timed with them first, and a plan of the march has to
+  // beat them.
   c->timing = false;
   c->iterations = kTuneIterations;
-  // what is tuned is the march's plan, for contexts that run it: a small
-  // volume that the cell kernels take stays theirs
-  c->tuning = true;
-  auto time_plan = [&](int w, int z, int u, float* ms) -> int {
+  auto time_plan = [&](int w, int z, int u, float* ms) -> int {  // u 0: the cell kernels
     c->flow_warps = w;
-    c->flow_units = u;
+    c->flow_units = std::max(1, u);
+    c->tuning = u > 0;  // the march, also where the cell kernels could run
     drop_graphs(c);
     int r = plan_flow(c, z);
     if (!r) r = hmf_solve(c, stream);
@@ -1920,6 +1931,12 @@ int hmf_autotune(hmf_ctx* c, void* stream) {
     if (!rc && ms < 2.0f)
       c->iterations = std::min(kTuneIterations * 32, (int)(kTuneIterations * std::ceil(2.0f / std::max(ms, 0.01f))));
   }
+  if (!rc && cells) {
+    float ms = 0;
+    const TunedPlan p{8, c->zchunk, 0};
+    rc = time_plan(p.warps, p.zchunk, p.units, &ms);
+    if (!rc) consider(ms, p);
+  }
   for (int w : {8, 16}) {
     if (rc) break;
     c->flow_warps = w;
@@ -1934,7 +1951,7 @@ int hmf_autotune(hmf_ctx* c, void* stream) {
     }
   }
   for (int u : {2, 4}) {
-    if (rc) break;
+    if (rc || best.units == 0) break;
     float ms = 0;
     rc = time_plan(best.warps, best.zchunk, u, &ms);
     if (!rc) consider(ms, TunedPlan{best.warps, best.zchunk, u});
@@ -1949,12 +1966,13 @@ int hmf_autotune(hmf_ctx* c, void* stream) {
   const TunedPlan& keep = rc ? before : best;
   drop_graphs(c);
   c->flow_warps = keep.warps;
-  c->flow_units = keep.units;
+  c->flow_units = std::max(1, keep.units);
+  c->march_tuned = rc ? saved_tuned : keep.units > 0;
   const int planned = plan_flow(c, keep.zchunk);
   if (rc) return rc;
   if (planned) return planned;
   std::lock_guard<std::mutex> lock(g_tune_mutex);
-  const std::string key = tune_key(c);
+  const std::string key = tune_key(c, cells);
   g_tune_cache[key] = best;
   tune_file_append(key, best);
   return HMF_OK;
@@ -1981,6 +1999,7 @@ int hmf_set_flow_window(hmf_ctx* c, int rows) {
   drop_graphs(c);
   c->flow_warps = rows == 64 ? 16 : 8;
   c->window_set = rows != 0;
+  c->march_tuned = false;
   c->zchunk_set = false;  // planned again
   return plan_flow(c, default_zchunk(c));
 }
@@ -1996,6 +2015,7 @@ int hmf_set_flow_units(hmf_ctx* c, int units) {
   drop_graphs(c);  // the captured launches carry the grid
   c->flow_units = units ? units : 1;
   c->units_set = units != 0;
+  c->march_tuned = false;
   return HMF_OK;
 }
 
@@ -2010,6 +2030,7 @@ int hmf_set_zchunk(hmf_ctx* c, int z) {
   int maxz = 1;
   for (const auto& V : c->vols) maxz = std::max(maxz, V.vz);
   c->zchunk_set = z != 0;
+  c->march_tuned = false;
   return plan_flow(c, z ? std::min(z, maxz) : default_zchunk(c));
 }
 

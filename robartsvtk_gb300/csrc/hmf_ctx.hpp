@@ -70,7 +70,8 @@ struct hmf_ctx {
   int zchunk = 0;  // planes per window column (0: not planned yet)
   int flow_warps = 8;  // flow_tma_kernel<W>: windows of 32 x 4W (hmf_set_flow_window)
   bool window_set = false, zchunk_set = false, units_set = false;  // chosen by the caller, each until set to 0
-  bool tuning = false;        // hmf_autotune times the march's plans
+  bool march_tuned = false;   // the plan is hmf_autotune's (or a saved one), faster than the cell kernels
+  bool tuning = false;        // hmf_autotune times a plan of the march
   bool overlap_launches = false;  // launches now recorded let the next kernel start early (launch_waiting)
   int flow_units = 1;  // flow_tma_kernel: (window, vertex) units marched by one CTA (hmf_set_flow_units)
   hmf::TreeTable* d_tree = nullptr;

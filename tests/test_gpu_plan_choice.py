@@ -2,6 +2,10 @@
 promise: settings that the caller made stay in force, the pipeline's getter says
 how the next solve runs, and a failed autotune changes nothing.  Results are the
 oracle's bit for bit on every route.  GPU only."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -12,6 +16,7 @@ from tests.test_gpu_parity import oracle
 pytestmark = pytest.mark.gpu
 
 TREE5 = [-1, 0, 0, 1, 1]
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def fill(s, w):
@@ -84,3 +89,46 @@ def test_a_window_restores_the_default_chunk():
         fill(s, w)
         s.solve()
         assert s.zchunk() == z and s.stats()["launches"] == 1 + 2 * w.iterations
+
+
+TUNED = """
+import sys
+from robartsvtk_gb300 import HMFSolver
+from robartsvtk_gb300.synthetic import random_tree_problem
+from tests.test_gpu_plan_choice import TREE5, assert_oracle, fill
+w = random_tree_problem(30, (40, 36, 28), TREE5, iterations=9, smooth_nodes=(1,))
+with HMFSolver(w.dims, w.parent) as s:
+    fill(s, w)
+    if "tune" in sys.argv:
+        s.autotune()
+    s.solve()
+    assert_oracle(s, w)
+    print("plan", s.flow_window, s.zchunk(), s.flow_units)
+"""
+
+
+def tuned_process(cache, *args):
+    """The plan of a context in a process of its own, which reads `cache`."""
+    env = dict(os.environ, HMF_AUTOTUNE_CACHE=str(cache))
+    r = subprocess.run([sys.executable, "-c", TUNED, *args], cwd=ROOT, env=env, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    return [int(x) for x in r.stdout.split("plan")[1].split()]
+
+
+def test_autotune_of_a_small_volume(tmp_path):
+    """The small volume's own kernels are a candidate, and its plans are cached
+    apart from plans that were not timed against them."""
+    cache = tmp_path / "tuned"
+    default = tuned_process(cache)
+    plan = tuned_process(cache, "tune")
+    key, *saved = cache.read_text().split()
+    assert key.startswith("cells/") and tuned_process(cache) == plan
+    if int(saved[2]) == 0:
+        assert plan == default
+    cache.write_text("%s 16 5 2\n" % key)
+    assert tuned_process(cache) == [64, 5, 2]
+    cache.write_text("%s 8 7 0\n" % key)  # the small volume's kernels won: the default plan
+    assert tuned_process(cache) == default
+    cache.write_text("%s 16 5 2\n" % key[len("cells/"):])  # tuned without them
+    assert tuned_process(cache) == default
