@@ -230,6 +230,13 @@ int build_dag(hmf_ctx* c, int n, int n_edges, const int* ep, const int* ec, cons
       const float t = (float)((c->e_weighted ? (double)c->e_weight[e] : 1.0) / c->n_parents[ec[e]]);
       c->wkids[v] += t * t;
     }
+  c->dag_reg_ok = n <= hmf::kDagRegMax;  // small graphs whose edges are all distinct
+  for (int v = 0; v < n; ++v) {
+    std::vector<int> parents;
+    for (int e : c->in_e[v]) parents.push_back(ep[e]);
+    std::sort(parents.begin(), parents.end());
+    if (std::adjacent_find(parents.begin(), parents.end()) != parents.end()) c->dag_reg_ok = false;
+  }
   return HMF_OK;
 }
 
@@ -291,6 +298,9 @@ int allocate_state(hmf_ctx* c) {
 long long flow_slots(const hmf_ctx* c) { return std::max(1, c->sm_count) * (c->flow_warps <= 8 ? 2LL : 1LL); }
 
 int flow_max_out_y(const hmf_ctx* c) { return 4 * c->flow_warps - 5; }
+
+// Whether a graph's sweep is dag_bulk_n_kernel.
+bool dag_in_parameters(const hmf_ctx* c) { return !c->dag_simple && !c->dag_generic && c->dag_reg_ok; }
 
 // Flow-kernel work plan for a given z-chunk length: windows of at most
 // 28 x (4W - 5) outputs spread evenly over each volume, z split into chunks
@@ -382,7 +392,7 @@ int default_zchunk(const hmf_ctx* c) {
   }
   // a wave covers about one row of windows only when one volume's chunk
   // takes many waves (a batch of small volumes puts whole volumes in a wave)
-  const bool pipelined = c->pipeline && c->vols.size() == 1 && (!c->dag || c->n <= hmf::kDagRegMax);
+  const bool pipelined = c->pipeline && c->vols.size() == 1 && (!c->dag || dag_in_parameters(c));
   const bool batched = c->pipeline && c->vols.size() > 1;
   const int cap = per_chunk > 8 * slots ? 24 : batched ? 96 : pipelined ? 64 : 48;
   const int third = (maxz + 2) / 3;
@@ -601,8 +611,8 @@ bool cells_possible(const hmf_ctx* c) {
 }
 
 bool cell_path(const hmf_ctx* c) {
-  return cells_possible(c) && default_flow(c) && !c->march_tuned && !c->tuning && c->pipeline && !c->gap_on &&
-         c->stall_kind < 0;
+  return cells_possible(c) && default_flow(c) && !c->march_tuned && !c->tuning && c->pipeline && !c->pipeline_asked &&
+         !c->gap_on && c->stall_kind < 0;
 }
 
 int launch_flow_cell(hmf_ctx* c, int parity, cudaStream_t s) {
@@ -745,9 +755,6 @@ int dag_grid(hmf_ctx* c, const void* kernel, size_t smem) {
   return (int)std::max<long long>(1, std::min<long long>(blocks, (long long)c->sm_count * per));
 }
 
-// Whether the graph's sweep is dag_bulk_n_kernel.
-bool dag_in_parameters(const hmf_ctx* c) { return !c->dag_simple && !c->dag_generic && c->dag_reg_ok; }
-
 // dag_bulk_n_kernel over the elements [base, base + vol).
 int launch_dag_elements(hmf_ctx* c, long long base, long long vol, cudaStream_t s) {
   const int smem = hmf::dag_bulk_n_smem_bytes(c->n);
@@ -869,9 +876,6 @@ bool slabs_possible(const hmf_ctx* c) {
   return c->h_fvol[0].zchunk >= 3;
 }
 
-// The pipeline as hmf_get_pipeline reports it: a label tree's.
-bool pipeline_active(const hmf_ctx* c) { return !c->dag && slabs_possible(c); }
-
 // On the default plan a single volume whose flow CTAs all fit on the GPU at
 // once is iterated in whole launches, each started while the previous one ends
 // (launch_waiting): one wave leaves no idle SMs for a slab's sweep, and every
@@ -880,10 +884,11 @@ bool pipeline_active(const hmf_ctx* c) { return !c->dag && slabs_possible(c); }
 // 72.0 against 66.6, 110 x 100 x 24 tree4 34.7 against 31.8, 128^3 with four
 // leaves (300 CTAs) 119.2 against 118.7, 70^3 with four leaves 36.0 against
 // 37.0; from the second wave on the pipeline wins (160 x 160 x 128, four
-// leaves: 157.1 against 175.6).
+// leaves: 157.1 against 175.6).  A label tree whose caller switched the pipeline
+// on is iterated in slabs at any size.
 bool slab_replay(const hmf_ctx* c) {
   if (!slabs_possible(c) || cell_path(c)) return false;
-  if (!default_flow(c) || c->vols.size() > 1) return true;
+  if (!default_flow(c) || c->vols.size() > 1 || (c->pipeline_asked && !c->dag)) return true;
   const long long units = (long long)c->n_items * (c->n - 1);
   return (units + c->flow_units - 1) / c->flow_units > flow_slots(c);
 }
@@ -1130,11 +1135,9 @@ int prepare_dag_table(hmf_ctx* c, cudaStream_t s, const Staged& in) {
     E.n_out = pout - E.first_out;
   }
   CK(cudaMemcpyAsync(c->d_dag, &T, sizeof(T), cudaMemcpyHostToDevice, s), "cudaMemcpyAsync(graph table)");
-  // the same graph as kernel parameters of dag_bulk_n_kernel (small graphs
-  // whose edges are all distinct)
+  // the same graph as kernel parameters of dag_bulk_n_kernel
   hmf::DagRegParams& R = c->h_dagreg;
   std::memset(&R, 0, sizeof(R));
-  c->dag_reg_ok = c->n <= hmf::kDagRegMax;
   for (int i = 0; i < c->n && c->dag_reg_ok; ++i) {
     const hmf::DagEntry& E = T.e[i];
     R.sink[i] = E.sink;
@@ -1146,7 +1149,6 @@ int prepare_dag_table(hmf_ctx* c, cudaStream_t s, const Staged& in) {
     R.n_in[i] = E.n_in;
     for (int j = 0; j < E.n_in; ++j) {
       const int p = T.in_parent[E.first_in + j];
-      if ((R.pmask[i] >> p) & 1u) c->dag_reg_ok = false;  // a repeated edge
       R.pmask[i] |= 1u << p;
       R.wup[i][p] = T.in_wup[E.first_in + j];
       R.wdown_ord[i][j] = T.in_wdown[E.first_in + j];
@@ -1981,14 +1983,14 @@ int hmf_autotune(hmf_ctx* c, void* stream) {
 int hmf_set_pipeline(hmf_ctx* c, int enabled) {
   if (!c) return HMF_ERR_INVALID_ARGUMENT;
   if (int rc = refuse_paged(c, "hmf_set_pipeline")) return rc;
-  if ((enabled != 0) == c->pipeline) return HMF_OK;
+  if ((enabled != 0) == c->pipeline && (enabled != 0) == c->pipeline_asked) return HMF_OK;
   DeviceGuard dg(c->device);
   drop_graphs(c);
-  c->pipeline = enabled != 0;
+  c->pipeline = c->pipeline_asked = enabled != 0;
   return HMF_OK;
 }
 
-int hmf_get_pipeline(const hmf_ctx* c) { return c ? (pipeline_active(c) ? 1 : 0) : HMF_ERR_INVALID_ARGUMENT; }
+int hmf_get_pipeline(const hmf_ctx* c) { return c ? (slab_replay(c) ? 1 : 0) : HMF_ERR_INVALID_ARGUMENT; }
 
 int hmf_set_flow_window(hmf_ctx* c, int rows) {
   if (!c) return HMF_ERR_INVALID_ARGUMENT;

@@ -94,6 +94,7 @@ struct hmf_ctx {
 
   // z-slab pipeline of the replayed iterations (hmf_set_pipeline)
   bool pipeline = true;
+  bool pipeline_asked = false;  // switched on by the caller
   int n_slabs = 0;         // segments: z slabs of a single volume, or groups of a batch's volumes
   int seg_neighbours = 1;  // slabs wait for the neighbouring slabs (1), volume groups for none (0)
   std::vector<int> seg_first_item, seg_items;  // flow work items of each segment
@@ -132,7 +133,7 @@ struct hmf_ctx {
   hmf::TreeTable h_tree{};
   hmf::DagTable h_dag{};
   hmf::DagRegParams h_dagreg{};
-  bool dag_reg_ok = false;  // h_dagreg describes the graph (<= 8 nodes, no repeated edge)
+  bool dag_reg_ok = false;  // h_dagreg can describe the graph (<= 8 nodes, no repeated edge)
   std::vector<const float*> h_smooth_list;
 
   // the staged inputs of the last solve (per vertex; for hmf_get_energy)

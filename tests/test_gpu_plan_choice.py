@@ -9,13 +9,14 @@ import sys
 import numpy as np
 import pytest
 
-from robartsvtk_gb300 import HMFError, HMFSolver
+from robartsvtk_gb300 import DAGSolver, HMFError, HMFSolver
 from robartsvtk_gb300.synthetic import random_tree_problem
 from tests.test_gpu_parity import oracle
 
 pytestmark = pytest.mark.gpu
 
 TREE5 = [-1, 0, 0, 1, 1]
+TREE15 = [-1, 0, 0, 1, 1, 2, 2, 3, 3, 4, 4, 5, 5, 6, 6]
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
@@ -132,3 +133,31 @@ def test_autotune_of_a_small_volume(tmp_path):
     assert tuned_process(cache) == default
     cache.write_text("%s 16 5 2\n" % key[len("cells/"):])  # tuned without them
     assert tuned_process(cache) == default
+
+
+@pytest.mark.parametrize("dims,parent,default", [((40, 30, 60), TREE5, False), ((64, 60, 48), TREE5, False),
+                                                 ((100, 80, 60), TREE15, True)])
+def test_the_pipeline_getter_says_how_the_next_solve_runs(dims, parent, default):
+    """A small volume's own kernels, one wave in whole launches, and slabs."""
+    w = random_tree_problem(31, dims, parent, iterations=5, smooth_nodes=(1,))
+    with HMFSolver(w.dims, w.parent) as s:
+        fill(s, w)
+        slabs = -(-dims[2] // s.zchunk())
+        for switch, expected in ((None, default), (True, slabs > 1), (False, False), (True, slabs > 1)):
+            if switch is not None:
+                s.set_pipeline(switch)
+            if slabs > 1:
+                assert s.pipeline == expected, switch
+            s.solve()
+            assert s.stats()["launches"] == 1 + 2 * (slabs if expected else 1) * w.iterations
+            assert_oracle(s, w, (dims, switch))
+
+
+def test_the_pipeline_getter_of_graphs():
+    edges = [(0, 1), (1, 2), (1, 3), (0, 4), (4, 5), (4, 6), (4, 3)]
+    for dims, more, pipelined in (((40, 30, 20), [], False), ((200, 200, 90), [], True),
+                                  ((200, 200, 90), [(4, 3)], False)):  # a repeated edge: the general sweep
+        with DAGSolver(dims, 7, edges + more) as s:
+            assert s.pipeline == pipelined
+            s.set_pipeline(False)
+            assert not s.pipeline
