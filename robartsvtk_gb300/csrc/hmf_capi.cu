@@ -606,7 +606,7 @@ bool default_flow(const hmf_ctx* c) { return !c->window_set && !c->zchunk_set &&
 
 // What the context is, whatever was set on it since.
 bool cells_possible(const hmf_ctx* c) {
-  return c->use_tma && c->tree_kind == 0 && !c->dag && c->vols.size() == 1 && c->n <= hmf::kSweepCellMax &&
+  return !c->kernels_named && !c->dag && c->vols.size() == 1 && c->n <= hmf::kSweepCellMax &&
          c->semantics == HMF_SEMANTICS_REF_CUDA && c->total * (c->n - 1) <= kCellVoxels;
 }
 
@@ -1552,11 +1552,15 @@ int create_context(hmf_ctx** out, int n_volumes, const int* dims, int semantics,
     c->dag_simple = std::strcmp(e, "simple") == 0;
     c->dag_generic = std::strcmp(e, "generic") == 0;
   }
-  // Kernel selection.  HMF_FLOW_KERNEL=ring / HMF_TREE_KERNEL=quad|scalar select
-  // the simpler kernels (same results), for comparisons.
-  if (const char* e = std::getenv("HMF_FLOW_KERNEL")) c->use_tma = std::strcmp(e, "ring") != 0 || n_volumes > 1;
+  // Kernel selection, for comparisons (same results).  HMF_FLOW_KERNEL=tma|ring
+  // and HMF_TREE_KERNEL=bulk|quad|scalar name the kernels, at any size.
+  if (const char* e = std::getenv("HMF_FLOW_KERNEL")) {
+    c->kernels_named = true;
+    c->use_tma = std::strcmp(e, "ring") != 0 || n_volumes > 1;
+  }
   c->tree_kind = 0;
   if (const char* e = std::getenv("HMF_TREE_KERNEL")) {
+    c->kernels_named = true;
     if (std::strcmp(e, "quad") == 0 && c->n <= hmf::kTree4MaxVertices) c->tree_kind = 1;
     if (std::strcmp(e, "scalar") == 0) c->tree_kind = 2;
   }

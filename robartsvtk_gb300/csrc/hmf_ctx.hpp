@@ -80,6 +80,7 @@ struct hmf_ctx {
   bool dag_simple = false;   // dag_sweep_kernel (HMF_DAG_KERNEL=simple)
   bool dag_generic = false;  // dag_bulk_kernel even for small graphs (HMF_DAG_KERNEL=generic)
   bool use_tma = true;  // flow_tma_kernel (else the shared-memory ring flow_kernel)
+  bool kernels_named = false;  // by HMF_FLOW_KERNEL or HMF_TREE_KERNEL
   int tree_kind = 0;    // 0 tree_bulk_kernel, 1 tree4_kernel, 2 tree_kernel
   const float** d_smooth_list = nullptr;
   int* d_error = nullptr;
