@@ -263,9 +263,9 @@ int hmf_get_flow_units(const hmf_ctx* ctx);
  * per-slab graph nodes that wait only for the slabs their stencil touches, so
  * sweeps overlap flows and consecutive iterations overlap.  Same arithmetic,
  * bit-identical results.  On by default, where a volume whose flow step is
- * resident on the GPU at once runs in whole launches all the same, and one of
- * at most 350,000 voxel-vertices in kernels of its own that no plan concerns;
- * switched on by the caller, or with a z chunk, window or units per CTA set by
+ * resident on the GPU at once runs in whole launches all the same, and a small
+ * one (at most 350,000 voxel-vertices in 8 vertices, not flat) in kernels of
+ * its own that no plan concerns; switched on by the caller, or with a z chunk, window or units per CTA set by
  * the caller, a label tree is pipelined at any size (chunks of 3 planes or
  * more).  hmf_get_pipeline returns 1 when the next solve runs pipelined. */
 int hmf_set_pipeline(hmf_ctx* ctx, int enabled);

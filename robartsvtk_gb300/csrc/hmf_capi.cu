@@ -420,6 +420,16 @@ int default_zchunk(const hmf_ctx* c) {
   return best_z;
 }
 
+// Steps of the longest chain of flow CTAs, one after another on an SM, of a
+// single volume's default plan.
+long long default_steps(const hmf_ctx* c) {
+  const auto& V = c->vols[0];
+  const int z = default_zchunk(c), chunks = (V.vz + z - 1) / z, oy = flow_max_out_y(c);
+  const long long ctas = (long long)((V.vx + hmf::kTmaMaxOutX - 1) / hmf::kTmaMaxOutX) * ((V.vy + oy - 1) / oy) *
+                         chunks * (c->n - 1);
+  return (ctas + flow_slots(c) - 1) / flow_slots(c) * (chunks == 1 ? V.vz + 3 : z + 5);
+}
+
 // cuTensorMapEncodeTiled, fetched through the runtime so that the library
 // needs no link-time dependency on the driver library.
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -595,19 +605,34 @@ int launch_flow_tma_items(hmf_ctx* c, const hmf::FlowVertexTMA* table, int parit
 // Small volumes run the cell kernels (hmf_cell.cuh): single label-tree volumes
 // of at most kCellVoxels voxel-vertices and 8 vertices, on the default flow
 // plan (a window, z chunk or units chosen by the caller keep the march), with
-// no convergence log and no stall requested of the copy pipelines.  The limit
-// lies where the two paths cross (time per iteration, three leaves: 24 x 20 x 16
-// 9.9 us against the march's 15.1, 40 x 36 x 28 11.8 against 20.9, 52 x 52 x 48
-// -- 389,000 -- 24.8 against 23.9, 64^3 35.9 against 31.3).
+// no convergence log and no stall requested of the copy pipelines.  Within that
+// limit what counts is the number of cells, whole or not, against the steps of
+// the march's longest chain of CTAs: a step takes as long as about 120 cells
+// (fitted on 230 pairs; us per iteration, cells and march).  Three leaves:
+// 24 x 20 x 16, 72 cells and 6 steps, 8.8 and 11.9; 40 x 36 x 28, 315 and 7, 11.2
+// and 17.8; 52 x 52 x 48, 1008 and 8, 24.8 and 23.9; 300 x 300 x 1, 2166 and 8,
+// 34.4 and 18.9; 200 x 200 x 1, 975 and 4, 18.5 and 12.8; 1 x 20000 x 1, 7500 and
+// 32, 101 and 62.  More vertices: 8 x 8 x 900 in 6, 1350 and 23, 28.1 and 39.4;
+// 100 x 100 x 5 in 7, 1274 and 7, 26.9 and 18.1.
 constexpr long long kCellVoxels = 350000;
+constexpr long long kCellsPerStep = 120;
+
+// CTAs of flow_cell_kernel.
+long long flow_cells(const hmf_ctx* c) {
+  const auto& V = c->vols[0];
+  auto cells = [](int v, int edge) { return (long long)((v + edge - 1) / edge); };
+  return cells(V.vx, hmf::kCellX) * cells(V.vy, hmf::kCellY) * cells(V.vz, hmf::kCellZ) * (c->n - 1);
+}
 
 // No part of the march's plan was chosen by the caller.
 bool default_flow(const hmf_ctx* c) { return !c->window_set && !c->zchunk_set && !c->units_set; }
 
 // What the context is, whatever was set on it since.
 bool cells_possible(const hmf_ctx* c) {
-  return !c->kernels_named && !c->dag && c->vols.size() == 1 && c->n <= hmf::kSweepCellMax &&
-         c->semantics == HMF_SEMANTICS_REF_CUDA && c->total * (c->n - 1) <= kCellVoxels;
+  if (c->kernels_named || c->dag || c->vols.size() != 1 || c->n > hmf::kSweepCellMax ||
+      c->semantics != HMF_SEMANTICS_REF_CUDA || c->total * (c->n - 1) > kCellVoxels)
+    return false;
+  return flow_cells(c) <= kCellsPerStep * c->default_steps;
 }
 
 bool cell_path(const hmf_ctx* c) {
@@ -1595,6 +1620,7 @@ int create_context(hmf_ctx** out, int n_volumes, const int* dims, int semantics,
     rc = allocate_state(c);
     if (!rc) rc = configure_kernels(c);
     if (!rc) {
+      c->default_steps = default_steps(c);
       int z = 0;
       {
         std::lock_guard<std::mutex> lock(g_tune_mutex);

@@ -68,6 +68,7 @@ struct hmf_ctx {
   hmf::FlowItem* d_items = nullptr;
   int n_items = 0;
   int zchunk = 0;  // planes per window column (0: not planned yet)
+  long long default_steps = 0;  // of the default plan's longest chain of CTAs (one volume)
   int flow_warps = 8;  // flow_tma_kernel<W>: windows of 32 x 4W (hmf_set_flow_window)
   bool window_set = false, zchunk_set = false, units_set = false;  // chosen by the caller, each until set to 0
   bool march_tuned = false;   // the plan is hmf_autotune's (or a saved one), faster than the cell kernels

@@ -161,3 +161,21 @@ def test_the_pipeline_getter_of_graphs():
             assert s.pipeline == pipelined
             s.set_pipeline(False)
             assert not s.pipeline
+
+
+@pytest.mark.parametrize("dims,cells", [((40, 36, 28), True), ((24, 20, 16), True), ((8, 8, 300), True),
+                                        ((64, 16, 60), True), ((300, 280, 1), False), ((200, 200, 1), False),
+                                        ((1, 9000, 1), False), ((52, 52, 32), False)])
+def test_small_volumes_by_their_cells(dims, cells, tmp_path):
+    """Whether a volume's own kernels are its default (the autotuner's key says
+    so) goes by whole and partial 16 x 8 x 4 cells, not by voxels: flat and
+    narrow volumes march.  On a GPU of 152 SMs, to which the line belongs."""
+    import torch
+    if torch.cuda.get_device_properties(0).multi_processor_count != 152:
+        pytest.skip("another number of SMs: another line")
+    code = TUNED.replace("(40, 36, 28)", str(dims))
+    env = dict(os.environ, HMF_AUTOTUNE_CACHE=str(tmp_path / "tuned"))
+    r = subprocess.run([sys.executable, "-c", code, "tune"], cwd=ROOT, env=env, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert (tmp_path / "tuned").read_text().startswith("cells/") == cells
