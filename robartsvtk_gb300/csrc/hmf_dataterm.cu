@@ -115,8 +115,8 @@ __device__ __forceinline__ unsigned block_extreme(unsigned v, unsigned* warps /*
   return v;
 }
 
-// mm[0] = key of the minimum, mm[1] = key of the maximum (NaN skipped, as
-// vtkDataArray's range ignores it).
+// mm[0] = complement of the minimum's key, mm[1] = key of the maximum, both from
+// zero (NaN skipped, as vtkDataArray's range ignores it).
 __global__ void range_kernel(const float* __restrict__ in, long long n, unsigned int* mm) {
   unsigned int lo = 0xffffffffu, hi = 0u;
   auto take = [&](float v) {
@@ -137,7 +137,7 @@ __global__ void range_kernel(const float* __restrict__ in, long long n, unsigned
   lo = block_extreme<false>(lo, warps);
   hi = block_extreme<true>(hi, warps);
   if (threadIdx.x == 0) {
-    atomicMin(&mm[0], lo);
+    atomicMax(&mm[0], ~lo);
     atomicMax(&mm[1], hi);
   }
 }
@@ -172,12 +172,20 @@ __host__ __device__ inline bool ff_safe(double d) {
 // float near the reciprocal of the centre and minus its logarithm.
 constexpr int kExpHalf = 12;
 constexpr int kLogCells = 64;
-struct TermTables {
+struct TermTables {  // the logistic in float-float
+  static constexpr bool kFast = true, kLogistic = true;
   float ln2[3];
   FFloat ln2_ff;
   FFloat exp_tab[2 * kExpHalf + 1];
   float log_inv[kLogCells];
   FFloat log_tab[kLogCells];
+};
+
+struct NoTables {  // the Gaussian's entropy in float-float
+  static constexpr bool kFast = true, kLogistic = false;
+};
+struct InDouble {  // double throughout
+  static constexpr bool kFast = false, kLogistic = false;
 };
 
 TermTables make_term_tables() {
@@ -235,10 +243,6 @@ __device__ __forceinline__ FFloat ff_log(FFloat a, const TermTables& T) {
 struct TermParams {
   int op, entropy, two;
   double k1, c1, k2, c2;
-  float value[2];  // constant and spike: the results (normalised)
-  float spike;     // the spike's K1 as a float (spike_on: K1 is a float)
-  int spike_on;
-  int fast;                // the float-float path's constants are in its range
   Split3 c1s, c2s;         // C1, C2
   FFloat k1s, k2s;         // Gaussian: 1/K1, 1/K2; logistic: K1, K2
   int normalize;           // 0 none, 1 by off and mul, 2 Gaussian entropy: by the range at `range`
@@ -255,29 +259,28 @@ struct TermNorm {
 
 // vtkImageDataTermExecute1 (:62-249) and vtkImageDataTermExecute2 (:255-390) in
 // the reference's double arithmetic.
-__device__ __noinline__ float term_double(const TermParams& P, float f1, float f2) {
+__device__ __noinline__ float logistic_double(const TermParams& P, float f1, float f2) {
   const double x1 = (double)f1, x2 = (double)f2;
-  double v;
-  if (P.op == HMF_DATA_TERM_LOGISTIC) {
-    const double a = 1.0 + exp(-(P.k1 * (x1 - P.c1)));
-    if (P.two) {
-      const double b = 1.0 + exp(-(P.k2 * (x2 - P.c2)));
-      v = P.entropy ? log(a * b) : 1.0 / (a * b);
-    } else {
-      v = P.entropy ? log(a) : 1.0 / a;
-    }
-  } else {
-    const double q1 = (x1 - P.c1) / P.k1;
-    if (P.two) {
-      const double q2 = (x2 - P.c2) / P.k2;
-      v = P.entropy ? 0.5 * q1 * q1 + 0.5 * q2 * q2 : exp(-0.5 * q1 * q1 - 0.5 * (q2 * q2));
-    } else {
-      v = P.entropy ? 0.5 * q1 * q1 : exp(-0.5 * q1 * q1);
-    }
-  }
-  return (float)v;
+  const double a = 1.0 + exp(-(P.k1 * (x1 - P.c1)));
+  if (!P.two) return (float)(P.entropy ? log(a) : 1.0 / a);
+  const double b = 1.0 + exp(-(P.k2 * (x2 - P.c2)));
+  return (float)(P.entropy ? log(a * b) : 1.0 / (a * b));
 }
-__device__ __noinline__ float norm_double(float o, double off, double mul) { return (float)(((double)o + off) * mul); }
+__device__ __forceinline__ float gaussian_in_double(const TermParams& P, float f1, float f2) {
+  const double x1 = (double)f1, x2 = (double)f2;
+  const double q1 = (x1 - P.c1) / P.k1;
+  if (!P.two) return (float)(P.entropy ? 0.5 * q1 * q1 : exp(-0.5 * q1 * q1));
+  const double q2 = (x2 - P.c2) / P.k2;
+  return (float)(P.entropy ? 0.5 * q1 * q1 + 0.5 * q2 * q2 : exp(-0.5 * q1 * q1 - 0.5 * (q2 * q2)));
+}
+__device__ __forceinline__ float norm_in_double(float o, double off, double mul) {
+  return (float)(((double)o + off) * mul);
+}
+// The same beside the float-float path, out of line.
+__device__ __noinline__ float gaussian_double(const TermParams& P, float f1, float f2) {
+  return gaussian_in_double(P, f1, f2);
+}
+__device__ __noinline__ float norm_double(float o, double off, double mul) { return norm_in_double(o, off, mul); }
 
 __device__ __forceinline__ bool in_range(float a, float lo, float hi) { return a >= lo && a <= hi; }
 
@@ -296,62 +299,78 @@ __device__ __forceinline__ FFloat ff_minus(float x, const Split3& c, bool& ok) {
 // tested with 2^-41; the logistic's 2^-38.6 with 2^-37: its exponential and
 // logarithm, and the double result's 2^-53 / e^z from rounding 1 + e^z, which
 // for an entropy keeps e^z above 2^-10.
-__device__ __forceinline__ bool term_fast(const TermParams& P, const TermTables& T, float x1, float x2, float& out) {
-  if (!P.fast) return false;
+//
+// With VOTE a warp takes it together (`valid`: the lane has a voxel): where one
+// of its voxels lies outside the forms' range all of them go to double at once,
+// instead of after the others.  That counts in images too small to hide it: a
+// logistic of 2^16 voxels of which most lie outside takes 12.3 us without, 10.3
+// with it; in large images the vote costs up to a tenth.
+template <bool VOTE, class Tables>
+__device__ __forceinline__ bool term_fast(const TermParams& P, const Tables& T, float x1, float x2, bool valid,
+                                          float& out) {
   bool ok = true;
   const FFloat t1 = ff_mul(ff_minus(x1, P.c1s, ok), P.k1s);
   FFloat t2{0.0f, 0.0f};
   if (P.two) t2 = ff_mul(ff_minus(x2, P.c2s, ok), P.k2s);
-  if (!ok) return false;
-  if (P.op == HMF_DATA_TERM_GAUSSIAN) {
-    FFloat v = ff_mul(t1, t1);
-    if (!(t1.h == 0.0f) && !in_range(fabsf(t1.h), 0x1p-30f, 0x1p30f)) return false;
-    if (P.two) {
-      if (!(t2.h == 0.0f) && !in_range(fabsf(t2.h), 0x1p-30f, 0x1p30f)) return false;
-      v = ff_sum(v, ff_mul(t2, t2));
+  if constexpr (Tables::kLogistic) {
+    ok = ok && fabsf(t1.h) <= 32.0f && fabsf(t2.h) <= 32.0f;
+    if (P.entropy) ok = ok && (P.two ? fminf(t1.h, t2.h) <= 4.8f : t1.h <= 6.9f);  // (the limits below)
+  } else {
+    ok = ok && (t1.h == 0.0f || in_range(fabsf(t1.h), 0x1p-30f, 0x1p30f)) &&
+         (t2.h == 0.0f || in_range(fabsf(t2.h), 0x1p-30f, 0x1p30f));
+  }
+  if (VOTE && !__all_sync(0xffffffffu, ok || !valid)) return !valid;
+  if (!valid) return true;
+  if (!VOTE && !ok) return false;
+  FFloat v;
+  if constexpr (Tables::kLogistic) {
+    const FFloat e1 = ff_exp(FFloat{-t1.h, -t1.l}, T);
+    FFloat a = ff_sum(e1, 1.0f);
+    if (P.two) a = ff_mul(a, ff_sum(ff_exp(FFloat{-t2.h, -t2.l}, T), 1.0f));
+    if (P.entropy) {
+      if (!P.two && e1.h < 0x1p-7f) {
+        if (!(e1.h >= 0x1p-10f)) return false;
+        v = ff_log1p(e1, FFloat{0.0f, 0.0f});
+      } else {
+        if (!(a.h >= 1.0f + 0x1p-7f)) return false;
+        v = ff_log(a, T);
+      }
+    } else {
+      const float r = 1.0f / a.h;
+      const FFloat e = ff_sum(ff_mul(a, -r), 1.0f);  // 1 - a r
+      v = ff_sum(ff_mul(e, r), r);
     }
+    return ff_rounds(v, 0x1p-37f, out);
+  } else {  // the Gaussian's entropy
+    v = ff_mul(t1, t1);
+    if (P.two) v = ff_sum(v, ff_mul(t2, t2));
     if (v.h == 0.0f) {
       out = 0.0f;
       return true;
     }
     return ff_rounds(FFloat{0.5f * v.h, 0.5f * v.l}, 0x1p-41f, out);
   }
-  if (!(fabsf(t1.h) <= 32.0f && fabsf(t2.h) <= 32.0f)) return false;
-  const FFloat e1 = ff_exp(FFloat{-t1.h, -t1.l}, T);
-  FFloat a = ff_sum(e1, 1.0f);
-  if (P.two) a = ff_mul(a, ff_sum(ff_exp(FFloat{-t2.h, -t2.l}, T), 1.0f));
-  FFloat v;
-  if (P.entropy) {
-    if (!P.two && e1.h < 0x1p-7f) {
-      if (!(e1.h >= 0x1p-10f)) return false;
-      v = ff_log1p(e1, FFloat{0.0f, 0.0f});
-    } else {
-      if (!(a.h >= 1.0f + 0x1p-7f)) return false;
-      v = ff_log(a, T);
-    }
-  } else {
-    const float r = 1.0f / a.h;
-    const FFloat e = ff_sum(ff_mul(a, -r), 1.0f);  // 1 - a r
-    v = ff_sum(ff_mul(e, r), r);
-  }
-  return ff_rounds(v, 0x1p-37f, out);
 }
 
-__device__ __forceinline__ float term_value(const TermParams& P, const TermTables& T, const TermNorm& N, float x1,
-                                            float x2) {
-  if (P.op == HMF_DATA_TERM_CONSTANT) return P.value[0];
-  if (P.op == HMF_DATA_TERM_SPIKE) return P.spike_on && x1 == P.spike ? P.value[0] : P.value[1];
-  float o;
-  if (!term_fast(P, T, x1, x2, o)) o = term_double(P, x1, x2);
-  if (!P.normalize) return o;
-  if (N.fast) {  // (o + off) * mul
-    const FFloat a = ff_sum(ff_two_sum(o, N.offs.h), FFloat{N.offs.m, N.offs.l});
-    if (a.h == 0.0f && a.l == 0.0f && N.mul > 0.0) return 0.0f;
-    const FFloat v = ff_mul(a, N.muls);
-    float r;
-    if (in_range(fabsf(a.h), 0x1p-40f, 0x1p40f) && ff_rounds(v, 0x1p-43f, r)) return r;
+template <bool VOTE, class Tables>
+__device__ __forceinline__ float term_value(const TermParams& P, const Tables& T, const TermNorm& N, float x1,
+                                            float x2, bool valid) {
+  float o = 0.0f;
+  if constexpr (!Tables::kFast) {
+    o = P.op == HMF_DATA_TERM_LOGISTIC ? logistic_double(P, x1, x2) : gaussian_in_double(P, x1, x2);
+    return P.normalize ? norm_in_double(o, N.off, N.mul) : o;
+  } else {
+    if (!term_fast<VOTE>(P, T, x1, x2, valid, o)) o = Tables::kLogistic ? logistic_double(P, x1, x2) : gaussian_double(P, x1, x2);
+    if (!P.normalize) return o;
+    if (N.fast) {  // (o + off) * mul
+      const FFloat a = ff_sum(ff_two_sum(o, N.offs.h), FFloat{N.offs.m, N.offs.l});
+      if (a.h == 0.0f && a.l == 0.0f && N.mul > 0.0) return 0.0f;
+      const FFloat v = ff_mul(a, N.muls);
+      float r;
+      if (in_range(fabsf(a.h), 0x1p-40f, 0x1p40f) && ff_rounds(v, 0x1p-43f, r)) return r;
+    }
+    return norm_double(o, N.off, N.mul);
   }
-  return norm_double(o, N.off, N.mul);
 }
 
 // Normalisation of a Gaussian entropy by the image's range [R0, R1]
@@ -367,44 +386,90 @@ __device__ __forceinline__ void gaussian_range_norm(const TermParams& P, double 
   mul = 1.0 / (mx - mn);
 }
 
+// Smallest images of the float-float forms, and of four voxels per thread in
+// them (Gaussian, logistic).  Below the first, launches cost what they cost:
+// us per call in double, float-float with a voxel and with four per thread,
+// Gaussian entropy of 4,000 voxels 6.2, 6.0, 6.1, of 131,072 7.4, 6.1, 6.2, of
+// 524,288 16.5, 7.3, 6.2; logistic entropy of 4,000 7.4, 6.0, 8.2, of 32,768 8.1,
+// 6.7, 8.3, of 262,144 28.7, 10.3, 10.3, of 524,288 51.4, 14.4, 12.4; one whose
+// voxels lie outside the float-float range of 16,384 7.7, 8.2, 20.6, of 262,144
+// 28.7, 28.8, 32.9.
+constexpr long long kTermFast[2] = {1 << 14, 1 << 15};
+constexpr long long kTermQuads[2] = {1 << 18, 1 << 19};
+
 // One voxel's result depends on it alone: bound by the arithmetic.  In double
 // throughout it kept the FP64 pipe 86 % busy (256 x 256 x 192, Gaussian entropy
 // normalised: 574 us; logistic entropy about as long); in float-float 89 us on
 // average, where its 15 us of traffic no longer matter either.
+//
+// Double throughout (InDouble) is for what has no float-float form, the
+// Gaussian's probability among it, and for small images.  It takes a voxel per
+// thread: four in one thread wait for one another's FP64.
+template <class Tables>
 __global__ void __launch_bounds__(kThreads) data_term_kernel(const __grid_constant__ TermParams P,
-                                                             const __grid_constant__ TermTables tables,
+                                                             const __grid_constant__ Tables tables,
                                                              const float* __restrict__ in1,
-                                                             const float* __restrict__ in2, long long n,
+                                                             const float* __restrict__ in2, long long n, int quads,
                                                              float* __restrict__ out) {
-  __shared__ TermTables T;
+  __shared__ Tables T;
   __shared__ TermNorm N;
-  if (P.op == HMF_DATA_TERM_LOGISTIC)  // read with an index that differs from lane to lane
-    for (int i = threadIdx.x; i < (int)(sizeof(TermTables) / 4); i += blockDim.x)
+  if constexpr (Tables::kLogistic)  // read with an index that differs from lane to lane
+    for (int i = threadIdx.x; i < (int)(sizeof(Tables) / 4); i += blockDim.x)
       reinterpret_cast<float*>(&T)[i] = reinterpret_cast<const float*>(&tables)[i];
   if (threadIdx.x == 0 && P.normalize) {
     N.off = P.off;
     N.mul = P.mul;
     if (P.normalize == 2)
-      gaussian_range_norm(P, (double)key_float(P.range[0]), (double)key_float(P.range[1]), N.off, N.mul);
-    N.fast = ff_safe(N.off) && ff_safe(N.mul) && N.mul != 0.0;
-    N.offs = split3(N.off);
-    N.muls = split2(N.mul);
+      gaussian_range_norm(P, (double)key_float(~P.range[0]), (double)key_float(P.range[1]), N.off, N.mul);
+    if (Tables::kFast) {
+      N.fast = ff_safe(N.off) && ff_safe(N.mul) && N.mul != 0.0;
+      N.offs = split3(N.off);
+      N.muls = split2(N.mul);
+    }
   }
-  __syncthreads();
-  const long long stride = (long long)gridDim.x * blockDim.x, t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (Tables::kLogistic || P.normalize) __syncthreads();
+  const long long stride = (long long)gridDim.x * blockDim.x, first = (long long)blockIdx.x * blockDim.x;
   const bool two = P.two != 0;
-  const bool quads = ((reinterpret_cast<uintptr_t>(in1) | reinterpret_cast<uintptr_t>(out) |
-                       (two ? reinterpret_cast<uintptr_t>(in2) : 0)) & 15) == 0;
   const long long nq = quads ? n / 4 : 0;
-  for (long long q = t; q < nq; q += stride) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(in1) + q);
-    const float4 b = two ? __ldg(reinterpret_cast<const float4*>(in2) + q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float x1[4] = {a.x, a.y, a.z, a.w}, x2[4] = {b.x, b.y, b.z, b.w}, o[4];
+  if constexpr (Tables::kFast) {
+    for (long long q = first + threadIdx.x; q < nq; q += stride) {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(in1) + q);
+      const float4 b = two ? __ldg(reinterpret_cast<const float4*>(in2) + q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      float x1[4] = {a.x, a.y, a.z, a.w}, x2[4] = {b.x, b.y, b.z, b.w}, o[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) o[j] = term_value(P, T, N, x1[j], x2[j]);
-    reinterpret_cast<float4*>(out)[q] = make_float4(o[0], o[1], o[2], o[3]);
+      for (int j = 0; j < 4; ++j) o[j] = term_value<false>(P, T, N, x1[j], x2[j], true);
+      reinterpret_cast<float4*>(out)[q] = make_float4(o[0], o[1], o[2], o[3]);
+    }
   }
-  for (long long i = 4 * nq + t; i < n; i += stride) out[i] = term_value(P, T, N, in1[i], two ? in2[i] : 0.0f);
+  if constexpr (Tables::kLogistic) {  // a block's threads run the same number of turns: their warps vote
+    for (long long i0 = 4 * nq + first; i0 < n; i0 += stride) {
+      const long long i = i0 + threadIdx.x;
+      const bool valid = i < n;
+      const float o = term_value<true>(P, T, N, valid ? in1[i] : 0.0f, valid && two ? in2[i] : 0.0f, valid);
+      if (valid) out[i] = o;
+    }
+  } else {
+    for (long long i = 4 * nq + first + threadIdx.x; i < n; i += stride)
+      out[i] = term_value<false>(P, T, N, in1[i], two ? in2[i] : 0.0f, true);
+  }
+}
+
+// The constant and the spike operation: one of two values, formed by the host
+// (without `in`: the first).
+__global__ void __launch_bounds__(kThreads) term_choice_kernel(const float* __restrict__ in, float spike, float hit,
+                                                               float miss, long long n, float* __restrict__ out) {
+  const long long stride = (long long)gridDim.x * blockDim.x, t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long nq = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 ? n / 4 : 0;
+  for (long long q = t; q < nq; q += stride) {
+    float4 o = make_float4(hit, hit, hit, hit);
+    if (in) {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(in) + q);
+      o = make_float4(a.x == spike ? hit : miss, a.y == spike ? hit : miss, a.z == spike ? hit : miss,
+                      a.w == spike ? hit : miss);
+    }
+    reinterpret_cast<float4*>(out)[q] = o;
+  }
+  for (long long i = 4 * nq + t; i < n; i += stride) out[i] = !in || in[i] == spike ? hit : miss;
 }
 
 struct LLParams {
@@ -710,8 +775,7 @@ int hmf_data_term(int op, int entropy, int normalize, double k1, double c1, doub
     const bool on_device = op == HMF_DATA_TERM_GAUSSIAN && P.entropy;
     if (ranged) {
       e = sc.alloc(&mm, 2);
-      if (e == cudaSuccess) e = cudaMemsetAsync(mm, 0xff, sizeof(unsigned int), s);
-      if (e == cudaSuccess) e = cudaMemsetAsync(mm + 1, 0, sizeof(unsigned int), s);
+      if (e == cudaSuccess) e = cudaMemsetAsync(mm, 0, 2 * sizeof(unsigned int), s);
       if (e == cudaSuccess) {
         range_kernel<<<std::min(grid_for((n_voxels + 3) / 4), kReduceBlocks), kThreads, 0, s>>>(d1, n_voxels, mm);
         e = cudaGetLastError();
@@ -722,7 +786,7 @@ int hmf_data_term(int op, int entropy, int normalize, double k1, double c1, doub
     }
     P.normalize = on_device ? 2 : 1;
     P.range = mm;
-    const double R0 = key_float(h[0]), R1 = key_float(h[1]);
+    const double R0 = key_float(~h[0]), R1 = key_float(h[1]);
     const double K1 = P.k1, C1 = P.c1;
     double off = 0.0, mul = 1.0 / C1;
     if (op == HMF_DATA_TERM_GAUSSIAN) {
@@ -752,24 +816,35 @@ int hmf_data_term(int op, int entropy, int normalize, double k1, double c1, doub
     P.mul = mul;
   }
   if (op == HMF_DATA_TERM_CONSTANT || op == HMF_DATA_TERM_SPIKE) {
-    const double v[2] = {P.c1, P.c2};
-    for (int j = 0; j < 2; ++j) {
-      P.value[j] = (float)v[j];
-      if (P.normalize) P.value[j] = (float)(((double)P.value[j] + P.off) * P.mul);
-    }
-    P.spike = (float)P.k1;
-    P.spike_on = (double)P.spike == P.k1;
+    float value[2] = {(float)P.c1, (float)P.c2};
+    if (P.normalize)
+      for (float& v : value) v = (float)(((double)v + P.off) * P.mul);
+    const float spike = (float)P.k1;
+    if (op == HMF_DATA_TERM_SPIKE && !((double)spike == P.k1)) value[0] = value[1];  // no float equals K1
+    term_choice_kernel<<<grid_for((n_voxels + 3) / 4), kThreads, 0, s>>>(op == HMF_DATA_TERM_SPIKE ? d1 : nullptr, spike,
+                                                                        value[0], value[1], n_voxels, dout);
   } else {
     const bool gauss = op == HMF_DATA_TERM_GAUSSIAN;
     P.c1s = split3(P.c1);
     P.c2s = split3(P.c2);
     P.k1s = split2(gauss ? 1.0 / P.k1 : P.k1);
     P.k2s = split2(gauss ? 1.0 / P.k2 : P.k2);
-    P.fast = (!gauss || P.entropy) && ff_safe(P.c1) && ff_safe(P.k1) && P.k1 != 0.0 &&
-             (!P.two || (ff_safe(P.c2) && ff_safe(P.k2) && P.k2 != 0.0));
+    // the constants are in the float-float forms' range
+    const bool fast = (!gauss || P.entropy) && ff_safe(P.c1) && ff_safe(P.k1) && P.k1 != 0.0 &&
+                      (!P.two || (ff_safe(P.c2) && ff_safe(P.k2) && P.k2 != 0.0));
+    const uintptr_t at = reinterpret_cast<uintptr_t>(d1) | reinterpret_cast<uintptr_t>(d2) | reinterpret_cast<uintptr_t>(dout);
+    const bool in_double = !fast || n_voxels < kTermFast[gauss ? 0 : 1];
+    const int quads = !in_double && n_voxels >= kTermQuads[gauss ? 0 : 1] && (at & 15) == 0;
+    const int grid = grid_for(quads ? (n_voxels + 3) / 4 : n_voxels);
+    if (in_double) {
+      data_term_kernel<<<grid, kThreads, 0, s>>>(P, InDouble{}, d1, d2, n_voxels, 0, dout);
+    } else if (gauss) {
+      data_term_kernel<<<grid, kThreads, 0, s>>>(P, NoTables{}, d1, d2, n_voxels, quads, dout);
+    } else {
+      static const TermTables tables = make_term_tables();
+      data_term_kernel<<<grid, kThreads, 0, s>>>(P, tables, d1, d2, n_voxels, quads, dout);
+    }
   }
-  static const TermTables tables = make_term_tables();
-  data_term_kernel<<<grid_for((n_voxels + 3) / 4), kThreads, 0, s>>>(P, tables, d1, d2, n_voxels, dout);
   e = cudaGetLastError();
   if (e == cudaSuccess && where == HMF_HOST) {
     e = cudaMemcpyAsync(out, dout, sizeof(float) * (size_t)n_voxels, cudaMemcpyDeviceToHost, s);
