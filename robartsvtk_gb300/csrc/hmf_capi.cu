@@ -371,7 +371,11 @@ int plan_flow(hmf_ctx* c, int zchunk) {
 // single wave in whole launches (slab_replay; 100 x 128 x 120 tree4, cost ratio
 // 0.93: 144.4 us whole, 126.0 in five slabs; 110^3 four leaves, 1.05: 96.1
 // and 91.7; 84 x 80 x 190 tree5, 1.11: 107.9 and 111.3; 168 x 162 x 62 four
-// leaves, 1.21: 90.9 and 95.9).
+// leaves, 1.21: 90.9 and 95.9).  A slab's two launches count for a quarter of a
+// step, so that long thin volumes are not cut into many (8 x 8 x 6000, three
+// leaves: 165 us in 200 slabs of a graph of 32 iterations, 846 in graphs of 8 and
+// 2, 100 whole; 112 x 108 x 500, two leaves: 163 in 19, 149 whole; 56 x 54 x 600
+// tree4: 153 in 25, 130 whole).
 //
 // A pipelined batch has no waves (its groups' launches overlap): what counts is
 // the planes marched and, a little, the longest march, with which a group's
@@ -413,7 +417,7 @@ int default_zchunk(const hmf_ctx* c) {
     }
     if (z > slab_cap && ctas > slots) continue;
     double cost = (double)((ctas + slots - 1) / slots) * (double)(z + 7);
-    if (slabs && ctas > slots) cost *= 0.9;
+    if (slabs && ctas > slots) cost = 0.9 * cost + 0.25 * chunks;
     if (batched) cost = (double)planes / (double)slots + 0.2 * (double)(z + 7);
     if (cost < best) best = cost, best_z = z;  // ties keep the longer chunk
   }

@@ -179,3 +179,16 @@ def test_small_volumes_by_their_cells(dims, cells, tmp_path):
                        timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
     assert (tmp_path / "tuned").read_text().startswith("cells/") == cells
+
+
+@pytest.mark.parametrize("dims,parent", [((8, 8, 6000), [-1, 0, 0, 0]), ((5, 30, 4700), [-1, 0, 0])])
+def test_a_long_thin_volume_is_not_cut_into_many_slabs(dims, parent):
+    import torch
+    if torch.cuda.get_device_properties(0).multi_processor_count != 152:
+        pytest.skip("another number of SMs: another plan")
+    w = random_tree_problem(33, dims, parent, iterations=3)
+    with HMFSolver(w.dims, w.parent) as s:
+        fill(s, w)
+        s.solve()
+        assert not s.pipeline and s.stats()["launches"] == 1 + 2 * w.iterations
+        assert_oracle(s, w, dims)
