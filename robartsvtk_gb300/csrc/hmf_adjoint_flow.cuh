@@ -39,6 +39,7 @@
 
 #include "hmf_async.cuh"
 #include "hmf_f32x2.cuh"
+#include "hmf_ff.cuh"
 #include "hmf_multiplier.cuh"
 #include "hmf_types.cuh"
 
@@ -85,17 +86,6 @@ struct AdjFlowParams {
   int* error_flag;
   unsigned long long wait_limit_ns;  // bound of every copy wait (kTmaWaitLimitNs unless a caller sets it)
 };
-
-// Float-float running sum: each term is added with Knuth's TwoSum, its rounding
-// error collected in lo.
-struct FF {
-  float hi, lo;
-};
-__device__ __forceinline__ void ff_accumulate(FF& a, float t) {
-  const float s = a.hi + t, b = s - a.hi;
-  a.lo += (a.hi - (s - b)) + (t - b);
-  a.hi = s;
-}
 
 __global__ void __launch_bounds__(kAfThreads, 1)
 adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowParams fp) {
@@ -391,7 +381,7 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
                 mv[j] = mj;
                 fv[j] = -mb * lj / (4.0f * Fm * Fm * Fm);
                 if (own && (j == 0 || in[1]) && (ST || kc >= zs) && kc < ze)
-                  ff_accumulate(asum, mb / Fm * (has_s ? (j ? f2_hi(S_c) : f2_lo(S_c)) : 1.0f));
+                  ff_add(asum, mb / Fm * (has_s ? (j ? f2_hi(S_c) : f2_lo(S_c)) : 1.0f));
               }
             }
           }
