@@ -92,7 +92,7 @@ adj_flow_tma_kernel(const AdjFlowVertex* __restrict__ vertices, const AdjFlowPar
   extern __shared__ __align__(1024) unsigned char af_raw[];
   float* mslots = reinterpret_cast<float*>(af_raw);                      // [3][10][1216]
   float* zslots = mslots + kAfMainSlots * kAfMainArrays * kAfPlane;      // [4][1216]
-  float* xp = zslots + kAfPzSlots * kAfPlane;                            // [11][34][32]
+  float* xp = zslots + kAfPzSlots * kAfPlane;                            // [14][34][32]
   uint64_t* mbars = reinterpret_cast<uint64_t*>(xp + kAfXPlanes * kAfX); // [3]
   uint64_t* zbars = mbars + kAfMainSlots;                                // [4]
   uint64_t* stall_bar = zbars + kAfPzSlots;                              // [1] never completed (a requested stall)

@@ -293,10 +293,10 @@ int allocate_state(hmf_ctx* c) {
   return HMF_OK;
 }
 
-// Output rows of one flow window of the context's shape.
 // Flow CTAs resident at once.
 long long flow_slots(const hmf_ctx* c) { return std::max(1, c->sm_count) * (c->flow_warps <= 8 ? 2LL : 1LL); }
 
+// Output rows of one flow window of the context's shape.
 int flow_max_out_y(const hmf_ctx* c) { return 4 * c->flow_warps - 5; }
 
 // Whether a graph's sweep is dag_bulk_n_kernel.
@@ -375,7 +375,11 @@ int plan_flow(hmf_ctx* c, int zchunk) {
 // step, so that long thin volumes are not cut into many (8 x 8 x 6000, three
 // leaves: 165 us in 200 slabs of a graph of 32 iterations, 846 in graphs of 8 and
 // 2, 100 whole; 112 x 108 x 500, two leaves: 163 in 19, 149 whole; 56 x 54 x 600
-// tree4: 153 in 25, 130 whole).
+// tree4: 153 in 25, 130 whole).  The halo planes of shorter chunks are work all
+// the same, so such slabs gain a little alone and lose with several solves in
+// flight (160 x 160 x 60, three leaves, one at a time and four: 73.6 and 69.7 in
+// five slabs, 74.9 and 51.5 whole; 100 x 128 x 120 tree4 124.6 and 122.6, 138.8 and
+// 103.3).
 //
 // A pipelined batch has no waves (its groups' launches overlap): what counts is
 // the planes marched and, a little, the longest march, with which a group's

@@ -399,8 +399,10 @@ constexpr long long kTermQuads[2] = {1 << 18, 1 << 19};
 
 // One voxel's result depends on it alone: bound by the arithmetic.  In double
 // throughout it kept the FP64 pipe 86 % busy (256 x 256 x 192, Gaussian entropy
-// normalised: 574 us; logistic entropy about as long); in float-float 89 us on
-// average, where its 15 us of traffic no longer matter either.
+// normalised: 574 us); in float-float 79 us a call, of which 38 are the
+// normalisation: the range's pass and every block's constants in double.  A
+// logistic entropy takes 157 us of FP32 arithmetic, a Gaussian probability, in
+// double still, 750.
 //
 // Double throughout (InDouble) is for what has no float-float form, the
 // Gaussian's probability among it, and for small images.  It takes a voxel per
