@@ -262,12 +262,13 @@ int hmf_get_flow_units(const hmf_ctx* ctx);
  * iteration's flow and sweep launches are cut at the flow plan's z chunks into
  * per-slab graph nodes that wait only for the slabs their stencil touches, so
  * sweeps overlap flows and consecutive iterations overlap.  Same arithmetic,
- * bit-identical results.  On by default, where a volume whose flow step is
- * resident on the GPU at once runs in whole launches all the same, and a small
- * one (at most 350,000 voxel-vertices in 8 vertices, not flat) in kernels of
- * its own that no plan concerns; switched on by the caller, or with a z chunk, window or units per CTA set by
- * the caller, a label tree is pipelined at any size (chunks of 3 planes or
- * more).  hmf_get_pipeline returns 1 when the next solve runs pipelined. */
+ * bit-identical results.  On by default, where on the default plan a volume
+ * whose flow step is resident on the GPU at once runs in whole launches all the
+ * same, and a small one (at most 350,000 voxel-vertices in 8 vertices, not
+ * flat) in kernels of its own that no plan concerns; with a z chunk, window or
+ * units per CTA set by the caller a volume is pipelined at any size (chunks of 3
+ * planes or more).  hmf_get_pipeline returns 1 when the next solve runs
+ * pipelined. */
 int hmf_set_pipeline(hmf_ctx* ctx, int enabled);
 int hmf_get_pipeline(const hmf_ctx* ctx);
 

@@ -644,8 +644,8 @@ bool cells_possible(const hmf_ctx* c) {
 }
 
 bool cell_path(const hmf_ctx* c) {
-  return cells_possible(c) && default_flow(c) && !c->march_tuned && !c->tuning && c->pipeline && !c->pipeline_asked &&
-         !c->gap_on && c->stall_kind < 0;
+  return cells_possible(c) && default_flow(c) && !c->march_tuned && !c->tuning && c->pipeline && !c->gap_on &&
+         c->stall_kind < 0;
 }
 
 int launch_flow_cell(hmf_ctx* c, int parity, cudaStream_t s) {
@@ -917,11 +917,10 @@ bool slabs_possible(const hmf_ctx* c) {
 // 72.0 against 66.6, 110 x 100 x 24 tree4 34.7 against 31.8, 128^3 with four
 // leaves (300 CTAs) 119.2 against 118.7, 70^3 with four leaves 36.0 against
 // 37.0; from the second wave on the pipeline wins (160 x 160 x 128, four
-// leaves: 157.1 against 175.6).  A label tree whose caller switched the pipeline
-// on is iterated in slabs at any size.
+// leaves: 157.1 against 175.6).
 bool slab_replay(const hmf_ctx* c) {
   if (!slabs_possible(c) || cell_path(c)) return false;
-  if (!default_flow(c) || c->vols.size() > 1 || (c->pipeline_asked && !c->dag)) return true;
+  if (!default_flow(c) || c->vols.size() > 1) return true;
   const long long units = (long long)c->n_items * (c->n - 1);
   return (units + c->flow_units - 1) / c->flow_units > flow_slots(c);
 }
@@ -2021,10 +2020,10 @@ int hmf_autotune(hmf_ctx* c, void* stream) {
 int hmf_set_pipeline(hmf_ctx* c, int enabled) {
   if (!c) return HMF_ERR_INVALID_ARGUMENT;
   if (int rc = refuse_paged(c, "hmf_set_pipeline")) return rc;
-  if ((enabled != 0) == c->pipeline && (enabled != 0) == c->pipeline_asked) return HMF_OK;
+  if ((enabled != 0) == c->pipeline) return HMF_OK;
   DeviceGuard dg(c->device);
   drop_graphs(c);
-  c->pipeline = c->pipeline_asked = enabled != 0;
+  c->pipeline = enabled != 0;
   return HMF_OK;
 }
 

@@ -96,7 +96,6 @@ struct hmf_ctx {
 
   // z-slab pipeline of the replayed iterations (hmf_set_pipeline)
   bool pipeline = true;
-  bool pipeline_asked = false;  // switched on by the caller
   int n_slabs = 0;         // segments: z slabs of a single volume, or groups of a batch's volumes
   int seg_neighbours = 1;  // slabs wait for the neighbouring slabs (1), volume groups for none (0)
   std::vector<int> seg_first_item, seg_items;  // flow work items of each segment
