@@ -615,15 +615,16 @@ int launch_flow_tma_items(hmf_ctx* c, const hmf::FlowVertexTMA* table, int parit
 // plan (a window, z chunk or units chosen by the caller keep the march), with
 // no convergence log and no stall requested of the copy pipelines.  Within that
 // limit what counts is the number of cells, whole or not, against the steps of
-// the march's longest chain of CTAs: a step takes as long as about 120 cells
+// the march's longest chain of CTAs: a step takes as long as about 125 cells
 // (fitted on 230 pairs; us per iteration, cells and march).  Three leaves:
 // 24 x 20 x 16, 72 cells and 6 steps, 8.8 and 11.9; 40 x 36 x 28, 315 and 7, 11.2
 // and 17.8; 52 x 52 x 48, 1008 and 8, 24.8 and 23.9; 300 x 300 x 1, 2166 and 8,
 // 34.4 and 18.9; 200 x 200 x 1, 975 and 4, 18.5 and 12.8; 1 x 20000 x 1, 7500 and
-// 32, 101 and 62.  More vertices: 8 x 8 x 900 in 6, 1350 and 23, 28.1 and 39.4;
-// 100 x 100 x 5 in 7, 1274 and 7, 26.9 and 18.1.
+// 32, 101 and 62.  Two leaves: 20000 x 1 x 1, 2500 and 20, 35.5 and 42.6.  Six and
+// seven: 8 x 8 x 900, 1350 and 23, 28.1 and 39.4; 100 x 100 x 5, 1274 and 7, 26.9
+// and 18.1.
 constexpr long long kCellVoxels = 350000;
-constexpr long long kCellsPerStep = 120;
+constexpr long long kCellsPerStep = 125;
 
 // CTAs of flow_cell_kernel.
 long long flow_cells(const hmf_ctx* c) {
